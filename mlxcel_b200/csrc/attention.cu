@@ -70,6 +70,16 @@ struct DecodeParams {
   int mean_of, mean_rows;
 };
 
+// Codes as floats: the code goes into the low mantissa bits of 2^23, which is then taken off (exact). An integer conversion
+// runs at an eighth of the rate of these two instructions: with it the decode kernel over an 8-bit pool took 50 us for 32 rows of
+// about 900 tokens and 8 key heads of 128, without it 41 us (62 MB: 10 us at the copy bandwidth).
+__device__ __forceinline__ float byte_to_float(uint32_t w, int j) {
+  return __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7650u | j)) - 8388608.0f;
+}
+__device__ __forceinline__ float nibble_to_float(uint32_t w, int j) {
+  return __uint_as_float(((w >> (4 * j)) & 0xFu) | 0x4B000000u) - 8388608.0f;
+}
+
 // Loads 8 consecutive elements of a K/V row as floats.
 template <int KV_BITS>
 __device__ __forceinline__ void load8(const void* pool, size_t elem_off, float (&f)[8]) {
@@ -85,12 +95,12 @@ __device__ __forceinline__ void load8(const void* pool, size_t elem_off, float (
     // two values per byte, even element in the low nibble: 8 elements = one 32-bit word
     const uint32_t w = *reinterpret_cast<const uint32_t*>(static_cast<const uint8_t*>(pool) + (elem_off >> 1));
 #pragma unroll
-    for (int j = 0; j < 8; ++j) f[j] = static_cast<float>((w >> (4 * j)) & 0xFu);
+    for (int j = 0; j < 8; ++j) f[j] = nibble_to_float(w, j);
   } else {
     const uint2 a = *reinterpret_cast<const uint2*>(static_cast<const uint8_t*>(pool) + elem_off);
     const uint32_t w[2] = {a.x, a.y};
 #pragma unroll
-    for (int j = 0; j < 8; ++j) f[j] = static_cast<float>((w[j >> 2] >> (8 * (j & 3))) & 0xFFu);
+    for (int j = 0; j < 8; ++j) f[j] = byte_to_float(w[j >> 2], j & 3);
   }
 }
 
@@ -860,11 +870,11 @@ paged_decode_mma_kernel(const DecodeParams p, const int heads_per_key) {
             const uint2 a = *reinterpret_cast<const uint2*>(codes + r * RAW_ROW + c * 8);
             const uint32_t w[2] = {a.x, a.y};
 #pragma unroll
-            for (int j = 0; j < 8; ++j) f[j] = static_cast<float>((w[j >> 2] >> (8 * (j & 3))) & 0xFFu);
+            for (int j = 0; j < 8; ++j) f[j] = byte_to_float(w[j >> 2], j & 3);
           } else {
             const uint32_t w = *reinterpret_cast<const uint32_t*>(codes + r * RAW_ROW + c * 4);
 #pragma unroll
-            for (int j = 0; j < 8; ++j) f[j] = static_cast<float>((w >> (4 * j)) & 0xFu);
+            for (int j = 0; j < 8; ++j) f[j] = nibble_to_float(w, j);
           }
           const uint32_t m = *reinterpret_cast<const uint32_t*>(meta + r * META_ROW + ((c * 8) / 64) * 4);
           const float sc = bf16_lo(m), bi = bf16_hi(m);
