@@ -316,6 +316,13 @@ int mx_read_status(void* workspace, int clear);
 const char* mx_build_info(void);
 
 
+// Attention of short pieces (a few query tokens per sequence, verify rounds) over long paged contexts: rows
+// [cu_q[s], cu_q[s + 1]) of q are the last tokens of sequence s. -10 = not covered.
+int mx_paged_verify(const void* q, long long q_stride, const void* k_pool, const void* v_pool, const void* k_meta, const void* v_meta,
+                    const int* block_tables, const int* cu_q, const int* context_lens, const float* sinks, void* out, void* scratch,
+                    int S, int max_q, int Hq, int Hkv, int D, int block_size, int max_blocks, int window, float scale, float softcap,
+                    int kv_bits, int num_splits, void* stream);
+
 // Grouped 4-bit GEMV over MLX-packed expert weights for decode-sized groups (few rows per expert).
 // -9 = shape not covered (the caller falls back to the grouped GEMM).
 int mx_moe_qgemv(const void* xs, const void* w, const void* scales, const void* biases, const void* lin_bias,

@@ -278,6 +278,10 @@ def paged_decode(q: torch.Tensor, kv: KVLayer, block_tables: torch.Tensor,
 
 
 _PREFILL_TC = os.environ.get("MLXCEL_B200_PREFILL_TC", "1") != "0"
+# Pieces of at most this many 16-row tiles per sequence and key head go through the decode kernel with their tokens packed. It
+# reads the context once per tile (about 50 us a layer and tile at 16 x 4090 tokens, 8 key heads), the tcgen05 kernel once, but
+# with one CTA per (128-row tile, key head): 571 us there whatever the pieces hold.
+_VERIFY_TILES = 4
 
 
 def paged_prefill(q: torch.Tensor, kv: KVLayer, block_tables: torch.Tensor, cu_q: torch.Tensor,
@@ -294,6 +298,23 @@ def paged_prefill(q: torch.Tensor, kv: KVLayer, block_tables: torch.Tensor, cu_q
     if T == 0:
         return out
     S = context_lens.shape[0]
+    pack = 16 // (Hq // Hkv) if Hq // Hkv <= 16 else 0        # query tokens of a sequence that share a 16-row tile
+    if pack and max_q_len <= _VERIFY_TILES * pack and kv.block_size == 16 and D in (64, 128) and q.stride(0) % 8 == 0 \
+            and q.dtype == torch.bfloat16 and (kv.kv_bits != 16 or kv.k.dtype == torch.bfloat16):
+        # verify rounds: a few query tokens per sequence over long contexts
+        tiles = -(-max_q_len // pack)
+        splits = decode_splits(S * tiles, Hkv, block_tables.shape[1] * kv.block_size)
+        lib = _lib.load()
+        floats = int(lib.mx_paged_decode_scratch_floats(S * tiles, Hkv * pack * (Hq // Hkv), D, splits)) if splits > 1 else 0
+        scratch = _decode_scratch(q.device, floats)
+        rc = lib.mx_paged_verify(q.data_ptr(), q.stride(0), kv.k.data_ptr(), kv.v.data_ptr(), _lib.ptr(kv.k_meta), _lib.ptr(kv.v_meta),
+                                 block_tables.data_ptr(), cu_q.data_ptr(), context_lens.data_ptr(), _lib.ptr(sinks), out.data_ptr(),
+                                 scratch.data_ptr(), S, max_q_len, Hq, Hkv, D, kv.block_size, block_tables.shape[1], window,
+                                 float(scale), float(softcap), kv.kv_bits, splits, _lib.stream())
+        if rc != -10:
+            _lib.count_launch()
+            _lib.check(rc, "mx_paged_verify")
+            return out
     if (_PREFILL_TC and kv.kv_bits == 16 and kv.block_size == 16 and D in (64, 128) and softcap == 0.0
             and kv.k.dtype == torch.bfloat16 and q.stride(0) % 8 == 0):
         # tensor-core (tcgen05) kernel; -10 = configuration not covered, fall through

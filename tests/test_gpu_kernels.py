@@ -264,6 +264,30 @@ def test_paged_prefill(Hq, Hkv, D, bits, window, sinks):
     _close(got, want, rtol=2e-2, atol=2e-2)
 
 
+@pytest.mark.parametrize("Hq,Hkv,D", [(8, 1, 128), (8, 2, 64), (4, 4, 64), (16, 1, 128), (12, 4, 128)])
+@pytest.mark.parametrize("bits,window,sinks", [(16, 0, False), (16, 40, True), (8, 0, True), (4, 24, False)])
+@pytest.mark.parametrize("ctx,qlen", [([5, 300, 33, 4, 17], [1, 4, 3, 4, 2]), ([1500], [4]), ([2, 16, 640], [2, 1, 7])])
+def test_paged_prefill_short_pieces(monkeypatch, Hq, Hkv, D, bits, window, sinks, ctx, qlen):
+    """Pieces of a few tokens share 16-row tiles of the decode kernel: tiles that are full, partly filled and empty, contexts that
+    end inside a key group or hold nothing but the piece, windows that begin inside a tile's tokens, key splits that are merged
+    (one sequence) and splits without keys."""
+    bs, nb = 16, 256
+    kv = _pool(nb, Hkv, bs, D, bits)
+    _fill_pool(kv, 6)
+    tab = _tables(ctx, bs, nb, 100)
+    cl = torch.tensor(ctx, dtype=torch.int32, device=DEV)
+    cu = torch.tensor([0] + list(torch.tensor(qlen).cumsum(0)), dtype=torch.int32, device=DEV)
+    q = _bf(sum(qlen), (Hq + 2 * Hkv) * D, seed=12)[:, : Hq * D]
+    sk = torch.randn(Hq, device=DEV) if sinks else None
+    kw = dict(Hq=Hq, Hkv=Hkv, D=D, scale=1.0 / math.sqrt(D), window=window, sinks=sk)
+    out = torch.full((sum(qlen), Hq * D), float("nan"), dtype=torch.bfloat16, device=DEV)
+    got = ops.paged_prefill(q, kv, tab, cu, cl, max_q_len=max(qlen), out=out, **kw)
+    _close(got, ref.paged_attention(q, kv, tab, cl, cu, **kw), rtol=2e-2, atol=2e-2)
+    # the kernels for longer pieces give the same
+    monkeypatch.setattr(ops, "_VERIFY_TILES", 0)
+    _close(got, ops.paged_prefill(q, kv, tab, cu, cl, max_q_len=max(qlen), **kw), rtol=2e-2, atol=2e-2)
+
+
 @pytest.mark.parametrize("M", [1, 16, 64, 200, 700])
 def test_gemm_deferred_rmsnorm(M):
     """producer GEMM (+residual) leaves per-tile sums of squares; consumer GEMMs (plain and gated)
