@@ -323,6 +323,10 @@ int mx_paged_verify(const void* q, long long q_stride, const void* k_pool, const
                     int S, int max_q, int Hq, int Hkv, int D, int block_size, int max_blocks, int window, float scale, float softcap,
                     int kv_bits, int num_splits, void* stream);
 
+// Gated projection of ONE row over affine 4-bit weights [2 * inter, K] (gate rows first). -9 = shape not covered.
+int mx_qmv_glu(const void* x, const void* w, const void* scales, const void* biases, void* out, const void* lin_bias, int inter, int K,
+               int group, int epi, float alpha, float limit, void* stream);
+
 // Grouped 4-bit GEMV over MLX-packed expert weights for decode-sized groups (few rows per expert).
 // -9 = shape not covered (the caller falls back to the grouped GEMM).
 int mx_moe_qgemv(const void* xs, const void* w, const void* scales, const void* biases, const void* lin_bias,

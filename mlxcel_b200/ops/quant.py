@@ -353,6 +353,18 @@ def qglu_linear(x: torch.Tensor, qt: QuantizedTensor, inter: int, act: str, bias
     from . import swiglu
 
     M, K = x.shape
+    if (x.is_cuda and M == 1 and _QMV_MAX_M >= 1 and qt.bits == 4 and qt.mode == "affine" and qt.packed.dim() == 2
+            and x.dtype == torch.bfloat16 and x.stride(1) == 1 and (bias is None or bias.dtype == torch.bfloat16)):
+        # one row: gate and up rows streamed once, activation in the epilogue (one launch)
+        from . import _ACT_TO_EPI
+        out = torch.empty(1, inter, dtype=torch.bfloat16, device=x.device)
+        rc = _lib.load().mx_qmv_glu(x.data_ptr(), qt.packed.data_ptr(), qt.scales.data_ptr(), qt.biases.data_ptr(), out.data_ptr(),
+                                    _lib.ptr(bias), inter, K, qt.group_size, _ACT_TO_EPI[act], float(alpha), float(limit),
+                                    _lib.stream())
+        if rc != -9:
+            _lib.count_launch()
+            _lib.check(rc, "mx_qmv_glu")
+            return out
     if (x.is_cuda and _QGEMV4 and 0 < M <= 8 and qt.bits == 4 and qt.mode in ("affine", "mxfp4") and qt.packed.dim() == 2
             and K % 32 == 0 and x.is_contiguous() and (bias is None or bias.dtype == torch.bfloat16)):
         # decode-sized: gate and up rows streamed once, activation in the epilogue (one launch)

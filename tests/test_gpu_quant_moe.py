@@ -45,6 +45,30 @@ def test_qlinear(mode, bits, group, M):
     _close(got.cpu(), want, rtol=2e-2, atol=6e-2)
 
 
+@pytest.mark.parametrize("N,K,group", [(1, 32, 32), (7, 1056, 32), (33, 2880, 64), (640, 4096, 64), (9475, 1024, 128)])
+def test_one_row_affine4(N, K, group):
+    """One row against affine 4-bit weights, plain (bias, residual) and gated: odd feature counts, rows of a single piece, a last
+    round that only some lanes take part in, both rows-per-warp forms. Everything is summed in fp32 (1e-5 of the sum of magnitudes
+    covers any order of it) and rounded once to bf16 (2^-8)."""
+    g = torch.Generator().manual_seed(N + K)
+    qt = _qt_to(quant.quantize(torch.randn(2 * N, K, generator=g) * 0.05, "affine", 4, group), DEV)
+    wd = quant.dequantize_ref(_qt_to(qt, "cpu")).double()
+    x = torch.randn(1, K, generator=g).to(torch.bfloat16)
+    bias = torch.randn(2 * N, generator=g).to(torch.bfloat16)
+    res = torch.randn(1, 2 * N, generator=g).to(torch.bfloat16)
+    y, size = x.double() @ wd.t(), x.double().abs() @ wd.abs().t()
+
+    def check(got, want, slack):
+        err = (got.cpu().double() - want).abs()
+        assert (err <= want.abs() * 2 ** -8 + slack * 1e-5 + 1e-6).all(), err.max().item()
+    check(quant.qlinear(x.to(DEV), qt), y, size)
+    check(quant.qlinear(x.to(DEV), qt, bias=bias.to(DEV), residual=res.to(DEV)), y + bias.double() + res.double(), size + 4)
+    z = y + bias.double()
+    want = torch.nn.functional.silu(z[:, :N]) * z[:, N:]
+    slack = (1.1 * size[:, :N] + 1) * (z[:, N:].abs() + 1) + z[:, :N].abs() * (size[:, N:] + 1)      # |silu'| < 1.1
+    check(quant.qglu_linear(x.to(DEV), qt, N, "silu", bias=bias.to(DEV)), want, slack)
+
+
 @pytest.mark.parametrize("mode,bits,group", [("affine", 4, 64), ("affine", 4, 128), ("affine", 8, 32), ("mxfp4", 4, 32)])
 @pytest.mark.parametrize("M", [1, 16, 64, 200])
 def test_fused_dequant_gemm(monkeypatch, mode, bits, group, M):
