@@ -339,17 +339,11 @@ def qgemm_graph():
             r = dict(M=M, N=N, K=K, packed_MB=round(packed_bytes / 1e6, 1),
                      stream_us_at_measured_copy_bw=round(packed_bytes / 6.5514e6, 1))
             old = quant._QMV_MAX_M
-            keep = quant._QGEMV4
-            if M <= 8:      # the grouped mma.sync weight-streaming kernel used as a dense GEMV (one group)
-                quant._QGEMV4 = True
-                r["gemv4_us"] = round(graph_time(lambda: [quant.qlinear(x, qts[i % ncopy], out=out) for i in range(nrep)]), 1)
-            quant._QGEMV4 = False
             quant._QMV_MAX_M = 0
             r["fused_qgemm_us"] = round(graph_time(lambda: [quant.qlinear(x, qts[i % ncopy], out=out) for i in range(nrep)]), 1)
             quant._QMV_MAX_M = old
-            if M <= 8:      # the older one-warp-per-row fp32 GEMV
+            if M <= 8:      # the fp32 GEMV kernels
                 r["qmv_us"] = round(graph_time(lambda: [quant.qlinear(x, qts[i % ncopy], out=out) for i in range(nrep)]), 1)
-            quant._QGEMV4 = keep
             quant._FUSED_QGEMM = False
             if M > 8:
                 r["dequant_then_gemm_us"] = round(

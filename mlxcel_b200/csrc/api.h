@@ -327,11 +327,10 @@ int mx_paged_verify(const void* q, long long q_stride, const void* k_pool, const
 int mx_qmv_glu(const void* x, const void* w, const void* scales, const void* biases, void* out, const void* lin_bias, int inter, int K,
                int group, int epi, float alpha, float limit, void* stream);
 
-// Grouped 4-bit GEMV over MLX-packed expert weights for decode-sized groups (few rows per expert).
+// Grouped 4-bit products over MLX-packed expert weights for decode-sized groups (few rows per expert).
 // -9 = shape not covered (the caller falls back to the grouped GEMM).
-int mx_moe_qgemv(const void* xs, const void* w, const void* scales, const void* biases, const void* lin_bias,
-                 const int* offsets, void* out, int E, int n_out, int K, int group, int mode, int epi,
-                 float alpha, float limit, const void* residual, long long ldo, long long ldr, void* stream);
+int mx_qstream(const void* xs, const void* w, const void* scales, const void* biases, const void* lin_bias, const int* offsets,
+               void* out, int E, int rows_used, int n_out, int K, int group, int mode, int epi, float alpha, float limit, void* stream);
 #ifdef __cplusplus
 }
 #endif

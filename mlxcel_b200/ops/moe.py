@@ -156,13 +156,12 @@ def grouped_linear(xs: torch.Tensor, w: torch.Tensor, offsets: torch.Tensor, n_o
         if (wq and _QGEMV_MAX_ROWS > 0 and used <= _QGEMV_MAX_ROWS * E and w.packed.dim() == 3 and K % 32 == 0
                 and (bias is None or bias.dtype == torch.bfloat16)):
             epi_gv = _ACT_TO_EPI[act] if act else (1 if bias is not None else 0)
-            rc = lib.mx_moe_qgemv(xs.data_ptr(), w.packed.data_ptr(), w.scales.data_ptr(), _lib.ptr(w.biases),
-                                  _lib.ptr(bias), offsets.data_ptr(), out.data_ptr(), E, n_out, K, w.group_size,
-                                  0 if w.mode == "affine" else 1, epi_gv, float(alpha), float(limit), None, 0, 0,
-                                  _lib.stream())
+            rc = lib.mx_qstream(xs.data_ptr(), w.packed.data_ptr(), w.scales.data_ptr(), _lib.ptr(w.biases), _lib.ptr(bias),
+                                offsets.data_ptr(), out.data_ptr(), E, used, n_out, K, w.group_size,
+                                0 if w.mode == "affine" else 1, epi_gv, float(alpha), float(limit), _lib.stream())
             if rc != -9:
                 _lib.count_launch()
-                _lib.check(rc, "mx_moe_qgemv")
+                _lib.check(rc, "mx_qstream")
                 return out
         expand = _DEQUANT_MIN_ROWS > 0 and used >= _DEQUANT_MIN_ROWS * E
         if wq and quant._FUSED_QGEMM and not expand and K % 64 == 0 and w.group_size in (32, 64, 128):

@@ -69,6 +69,34 @@ def test_one_row_affine4(N, K, group):
     check(quant.qglu_linear(x.to(DEV), qt, N, "silu", bias=bias.to(DEV)), want, slack)
 
 
+@pytest.mark.parametrize("mode,group", [("mxfp4", 32), ("affine", 32), ("affine", 64), ("affine", 128)])
+@pytest.mark.parametrize("counts,n_out,K", [([1], 16, 32), ([0, 9, 1, 40], 130, 2880), ([3, 0, 0, 0, 0, 0, 0, 2], 72, 1152),
+                                            ([17, 33, 8, 16], 64, 640)])
+@pytest.mark.parametrize("act", [None, "clipped_swiglu"])
+def test_expert_streaming_shapes(monkeypatch, mode, group, counts, n_out, K, act):
+    """Grouped 4-bit streaming products: scales that start inside a 32-bit word, a last block that is not full, K split over a
+    cluster, experts without rows and with several passes, every column-tile form, features that do not fill a warp's tile."""
+    if K % group:
+        pytest.skip("rows are whole groups")
+    monkeypatch.setattr(moe_ops, "_QGEMV_MAX_ROWS", 1 << 20)
+    g = torch.Generator().manual_seed(K + n_out)
+    E, rows = len(counts), sum(counts)
+    w = torch.randn(E, n_out * (2 if act else 1), K, generator=g) * 0.05
+    qt = quant.quantize(w, mode, 4, group)
+    wd = quant.dequantize_ref(qt)
+    xs = torch.randn(rows, K, generator=g).to(torch.bfloat16)
+    off = torch.tensor([0] + list(torch.tensor(counts).cumsum(0)), dtype=torch.int32)
+    b = (torch.randn(E, w.shape[1], generator=g) * 0.1).to(torch.bfloat16)
+    got = moe_ops.grouped_linear(xs.to(DEV), _qt_to(qt, DEV), off.to(DEV), n_out, b.to(DEV), act).cpu()
+    for e in range(E):
+        s = slice(int(off[e]), int(off[e + 1]))
+        z = xs[s].float() @ wd[e].t() + b[e].float()
+        if act:
+            from mlxcel_b200.ops import reference as ref
+            z = ref.glu_act(moe_ops._ACT_TO_EPI[act], z[:, :n_out], z[:, n_out:], 1.702, 7.0)
+        _close(got[s], z, rtol=1e-2, atol=1e-2)
+
+
 @pytest.mark.parametrize("mode,bits,group", [("affine", 4, 64), ("affine", 4, 128), ("affine", 8, 32), ("mxfp4", 4, 32)])
 @pytest.mark.parametrize("M", [1, 16, 64, 200])
 def test_fused_dequant_gemm(monkeypatch, mode, bits, group, M):
