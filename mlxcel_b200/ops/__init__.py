@@ -298,14 +298,16 @@ def paged_prefill(q: torch.Tensor, kv: KVLayer, block_tables: torch.Tensor, cu_q
     if T == 0:
         return out
     S = context_lens.shape[0]
-    pack = 16 // (Hq // Hkv) if Hq // Hkv <= 16 else 0        # query tokens of a sequence that share a 16-row tile
+    G = Hq // Hkv
+    # query tokens of a sequence that share a 16-row tile (for the calls that the kernels for longer pieces take too)
+    pack = 16 // G if G <= 16 and (G in (1, 2, 4, 8) or (_PREFILL_TC and kv.kv_bits == 16 and softcap == 0.0)) else 0
     if pack and max_q_len <= _VERIFY_TILES * pack and kv.block_size == 16 and D in (64, 128) and q.stride(0) % 8 == 0 \
             and q.dtype == torch.bfloat16 and (kv.kv_bits != 16 or kv.k.dtype == torch.bfloat16):
         # verify rounds: a few query tokens per sequence over long contexts
         tiles = -(-max_q_len // pack)
         splits = decode_splits(S * tiles, Hkv, block_tables.shape[1] * kv.block_size)
         lib = _lib.load()
-        floats = int(lib.mx_paged_decode_scratch_floats(S * tiles, Hkv * pack * (Hq // Hkv), D, splits)) if splits > 1 else 0
+        floats = int(lib.mx_paged_decode_scratch_floats(S * tiles, Hkv * pack * G, D, splits)) if splits > 1 else 0
         scratch = _decode_scratch(q.device, floats)
         rc = lib.mx_paged_verify(q.data_ptr(), q.stride(0), kv.k.data_ptr(), kv.v.data_ptr(), _lib.ptr(kv.k_meta), _lib.ptr(kv.v_meta),
                                  block_tables.data_ptr(), cu_q.data_ptr(), context_lens.data_ptr(), _lib.ptr(sinks), out.data_ptr(),

@@ -271,6 +271,8 @@ def test_paged_prefill_short_pieces(monkeypatch, Hq, Hkv, D, bits, window, sinks
     """Pieces of a few tokens share 16-row tiles of the decode kernel: tiles that are full, partly filled and empty, contexts that
     end inside a key group or hold nothing but the piece, windows that begin inside a tile's tokens, key splits that are merged
     (one sequence) and splits without keys."""
+    if bits != 16 and Hq // Hkv not in (1, 2, 4, 8):
+        pytest.skip("quantized pools are read for 1, 2, 4 or 8 query heads a key head")
     bs, nb = 16, 256
     kv = _pool(nb, Hkv, bs, D, bits)
     _fill_pool(kv, 6)
