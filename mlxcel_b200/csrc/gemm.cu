@@ -26,6 +26,7 @@
 
 #include "api.h"
 #include "common.cuh"
+#include "gemm_pair.cuh"
 
 namespace mx {
 
@@ -1906,6 +1907,20 @@ extern "C" int mx_gemm_bf16(const void* x, const void* w, void* out, const void*
   const int grid = static_cast<int>(total < cap ? total : cap);
 
   CUtensorMap map_x, map_w;
+  if (!swap && force_mode == 0 && !out_fp32) {
+    GemmPairParams pp{};
+    pp.out = static_cast<__nv_bfloat16*>(out);
+    pp.bias = p.bias, pp.residual = p.residual, pp.status = p.status;
+    pp.M = M, pp.N = N, pp.K = K, pp.ldo = ldo, pp.ldr = p.residual != nullptr ? ldr : 0;
+    pp.glu_offset = glu_offset, pp.epilogue = epilogue, pp.glu_alpha = glu_alpha, pp.glu_limit = glu_limit;
+    pp.ssq_in = p.ssq_in, pp.ssq_out = p.ssq_out, pp.ssq_eps = p.ssq_eps, pp.ssq_inv_dim = p.ssq_inv_dim;
+    if (gemm_pair_wanted(pp, glu, sms)) {
+      if (!make_tensor_map_bf16(&map_x, x, M, K, ldx, kLaneRows, kBK) ||
+          !make_tensor_map_bf16(&map_w, w, w_rows, K, ldw, kLaneRows, kBK))
+        return -4;
+      return gemm_pair_launch(map_x, map_w, pp, glu, sms, stream);
+    }
+  }
   const uint32_t x_box = swap ? bn : kLaneRows;
   const uint32_t w_box = swap ? kLaneRows : bn;
   if (!make_tensor_map_bf16(&map_x, x, M, K, ldx, x_box, kBK)) return -4;

@@ -290,6 +290,29 @@ def test_paged_prefill_short_pieces(monkeypatch, Hq, Hkv, D, bits, window, sinks
     _close(got, ops.paged_prefill(q, kv, tab, cu, cl, max_q_len=max(qlen), **kw), rtol=2e-2, atol=2e-2)
 
 
+@pytest.mark.parametrize("M,N,K", [(257, 264, 8), (512, 512, 512), (600, 136, 200), (1000, 1032, 1000), (2304, 4096, 448)])
+@pytest.mark.parametrize("form", ["plain", "bias", "residual", "gated"])
+def test_gemm_on_sm_pairs(M, N, K, form):
+    """Many-row projections on pairs of SMs: ragged rows, features and K, one k-slice, several tiles a pair, a single pair; against
+    64 bits, rounded once to bf16 (2^-8), with 1e-5 of the magnitudes for the order of the sums (gated: and for fast exp)."""
+    x, w = _bf(M, K, seed=1), _bf(2 * N if form == "gated" else N, K, seed=2, scale=0.05)
+    b = _bf(w.shape[0], seed=3) if form in ("bias", "gated") else None
+    res = _bf(M, N, seed=4) if form == "residual" else None
+    z = x.double() @ w.double().t() + (0 if b is None else b.double())
+    size = x.double().abs() @ w.double().abs().t() + 4
+    if form == "gated":
+        got = ops.glu_linear(x, w, N, "silu", bias=b)
+        size = 1.1 * size[:, :N] * (z[:, N:].abs() + 1) + z[:, :N].abs() * size[:, N:]      # |silu'| < 1.1
+        z = torch.nn.functional.silu(z[:, :N]) * z[:, N:]
+    else:
+        got = ops.linear(x, w, bias=b, residual=res)
+        z = z if res is None else z + res.double()
+    err = (got.double() - z).abs()
+    assert (err <= z.abs() * 2 ** -8 + size * 1e-5 + 1e-6).all(), err.max().item()
+    from mlxcel_b200.ops import _lib
+    assert _lib.read_status(torch.device(DEV)) == 0
+
+
 @pytest.mark.parametrize("M", [1, 16, 64, 200, 700])
 def test_gemm_deferred_rmsnorm(M):
     """producer GEMM (+residual) leaves per-tile sums of squares; consumer GEMMs (plain and gated)
