@@ -232,6 +232,24 @@ def fused_wq(qt: QuantizedTensor, M: int, K: int) -> int:
     return _FUSED_WQ.get((qt.mode, qt.bits), 0)
 
 
+def _paired_codes(by: torch.Tensor, qt: QuantizedTensor) -> torch.Tensor:
+    """Packed bytes of an affine 4-bit matrix with the eight codes of every 32-bit word in the order the GEMM's transform warps
+    take them apart: codes 0, 2, 4, 6 in the low half, 1, 3, 5, 7 in the high half. Other formats keep their order."""
+    if qt.bits != 4 or qt.mode != "affine":
+        return by
+    words = by.view(torch.int32)
+    out = torch.empty_like(words)
+
+    def squeeze(t):                       # the low nibbles of the four bytes, side by side
+        t = t & 0x0F0F0F0F
+        t = (t | (t >> 4)) & 0x00FF00FF
+        return (t | (t >> 8)) & 0xFFFF
+    # (in slices: the temporaries stay small next to the matrix)
+    for w, o in zip(words.view(-1).split(1 << 22), out.view(-1).split(1 << 22)):
+        torch.bitwise_or(squeeze(w), squeeze(w >> 4) << 16, out=o)
+    return out.view(torch.uint8)
+
+
 def tile_for_gemm(qt: QuantizedTensor) -> torch.Tensor:
     """Re-tile a 2-D quantized matrix for the fused dequant GEMM (built once, cached on the tensor).
 
@@ -241,7 +259,7 @@ def tile_for_gemm(qt: QuantizedTensor) -> torch.Tensor:
     (row tile, k-block) as ONE contiguous block that a single TMA box brings in:
 
         uint8 [T, K/64, 128 + E, W]    W = 64*bits/8 bytes per row, T = ceil(N / 128) (zero-padded)
-        rows 0..127   packed values of the 128 weight rows
+        rows 0..127   packed values of the 128 weight rows (affine 4-bit: see :func:`_paired_codes`)
         rows 128..    scales [2 halves of the k-block][128 rows], then biases likewise (affine),
                       bf16 (affine) or e8m0 bytes (mxfp4)
     """
@@ -252,7 +270,7 @@ def tile_for_gemm(qt: QuantizedTensor) -> torch.Tensor:
     bits, group = qt.bits, qt.group_size
     T, nkb, W = (N + 127) // 128, K // 64, 64 * bits // 8
     pad = T * 128 - N
-    by = qt.packed.contiguous().view(torch.uint8).view(N, nkb, W)
+    by = _paired_codes(qt.packed.contiguous().view(torch.uint8), qt).view(N, nkb, W)
     if pad:
         by = torch.cat([by, torch.zeros(pad, nkb, W, dtype=torch.uint8, device=by.device)], 0)
     vals = by.view(T, 128, nkb, W).permute(0, 2, 1, 3)                     # [T, nkb, 128, W]
@@ -287,7 +305,7 @@ def tile_experts_for_gemm(qt: QuantizedTensor, glu_inter: int | None = None) -> 
     bits, group = qt.bits, qt.group_size
     nkb, W = K // 64, 64 * bits // 8
     parts = [(0, N)] if glu_inter is None else [(0, glu_inter), (glu_inter, 2 * glu_inter)]
-    by = qt.packed.contiguous().view(torch.uint8).view(E, N, nkb, W)
+    by = _paired_codes(qt.packed.contiguous().view(torch.uint8), qt).view(E, N, nkb, W)
     halves = torch.arange(2 * nkb, device=by.device) * 32 // group
 
     def half_bytes(v, r0, r1, pad):   # [E, N, K/group] -> [E, T, nkb, bytes]
