@@ -36,11 +36,11 @@ NVCC_FLAGS = [
 # Sources a model family needs, for processes that serve one model from a tree without a built library:
 # they compile these alone, into a library of their own (the full one is used where it exists).
 MODEL_UNITS = {
-    "fusolix": ("attention", "attention_tc", "block_means", "gemm", "gemm_pair", "misc", "moe", "retention", "retention_tc", "sampling", "simt",
+    "fusolix": ("attention", "attention_tc", "attention_tc2", "block_means", "gemm", "gemm_pair", "misc", "moe", "retention", "retention_tc", "sampling", "simt",
                 "stream_norm", "streams"),
-    "govopel": ("attention", "attention_tc", "gemm", "gemm_pair", "latent", "latent_tc", "misc", "rope_norm", "sampling", "simt", "stream_norm"),
-    "pamasun": ("attention", "attention_tc", "delta_rule", "gemm", "gemm_pair", "misc", "sampling", "simt", "stream_norm"),
-    "vavadra": ("attention", "attention_tc", "gated_delta", "gemm", "gemm_pair", "latent", "latent_tc", "misc", "moe", "sampling", "simt", "stream_norm"),
+    "govopel": ("attention", "attention_tc", "attention_tc2", "gemm", "gemm_pair", "latent", "latent_tc", "misc", "rope_norm", "sampling", "simt", "stream_norm"),
+    "pamasun": ("attention", "attention_tc", "attention_tc2", "delta_rule", "gemm", "gemm_pair", "misc", "sampling", "simt", "stream_norm"),
+    "vavadra": ("attention", "attention_tc", "attention_tc2", "gated_delta", "gemm", "gemm_pair", "latent", "latent_tc", "misc", "moe", "sampling", "simt", "stream_norm"),
 }
 
 

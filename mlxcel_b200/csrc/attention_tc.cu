@@ -20,6 +20,7 @@
 // Replaces the reference's cuDNN SDPA prefill (mlx/backend/cuda/scaled_dot_product_attention.cpp in
 // its MLX overlay) and `chunked_causal_attention` (src/lib/mlxcel-core/src/layers.rs:5798).
 #include "api.h"
+#include "attention_tc2.cuh"
 #include "common.cuh"
 
 namespace mx {
@@ -710,6 +711,11 @@ extern "C" int mx_paged_prefill_tc(const void* q, long long q_stride, const void
   const uint64_t pool_rows = static_cast<uint64_t>(pool_blocks) * Hkv * kTcBlock;
   if (!make_tensor_map_bf16(&mk, k_pool, pool_rows, D, D, kTcBlock, 64)) return -4;
   if (!make_tensor_map_bf16(&mv, v_pool, pool_rows, D, D, kTcBlock, 64)) return -4;
+  if (Hq / Hkv % 2 == 0 && scale > 0.f) {
+    // two query heads of a key head per CTA; with an odd number of them (1 for plain multi-head attention) one
+    PrefillTc2Params t{block_tables, cu_q, context_lens, sinks, p.out, p.status, num_seqs, Hq, Hkv, max_blocks, window, p.tiles_per_seq, p.scale_log2};
+    return prefill_tc2_launch(mq, mk, mv, t, D, static_cast<int>(grid / 2), stream);
+  }
   if (D == 64) return launch_prefill_tc<64, 64, false>(mq, mk, mv, mv, mv, p, static_cast<int>(grid), stream);
   return launch_prefill_tc<128, 128, false>(mq, mk, mv, mv, mv, p, static_cast<int>(grid), stream);
 }

@@ -347,6 +347,29 @@ def test_gemm_deferred_rmsnorm(M):
     _close(ops.linear(h, fold(w2), row_norm=rn), ref.linear(x, w2, None, None), rtol=3e-2, atol=3e-2)
 
 
+@pytest.mark.parametrize("Hq,Hkv,D", [(2, 1, 128), (8, 2, 128), (4, 2, 64), (16, 1, 64), (6, 1, 128)])
+@pytest.mark.parametrize("ctx,qlen,window,sinks", [([128, 129, 700], [128, 129, 257], 0, False), ([1500, 127], [1000, 127], 0, True),
+                                                   ([900, 300, 1], [300, 300, 1], 130, True), ([2300], [260], 1, False)])
+def test_paged_prefill_two_heads(Hq, Hkv, D, ctx, qlen, window, sinks):
+    """Two query heads of a key head per CTA: one key tile and many, tiles that end on an edge, behind it and inside a row, a single
+    row, windows of one key and across tiles, large logits that move the running maximum by more than the rescaling threshold."""
+    bs, nb = 16, 512
+    kv = _pool(nb, Hkv, bs, D, 16)
+    _fill_pool(kv, 7)
+    tab = _tables(ctx, bs, nb, 160)
+    cl = torch.tensor(ctx, dtype=torch.int32, device=DEV)
+    cu = torch.tensor([0] + list(torch.tensor(qlen).cumsum(0)), dtype=torch.int32, device=DEV)
+    qkv = _bf(sum(qlen), (Hq + 2 * Hkv) * D, seed=11)
+    qkv[::37] *= 6.0
+    q = qkv[:, : Hq * D]
+    kw = dict(Hq=Hq, Hkv=Hkv, D=D, scale=1.0 / math.sqrt(D), window=window, sinks=torch.randn(Hq, device=DEV) if sinks else None)
+    out = torch.full((sum(qlen), Hq * D), float("nan"), dtype=torch.bfloat16, device=DEV)
+    got = ops.paged_prefill(q, kv, tab, cu, cl, max_q_len=max(qlen), out=out, **kw)
+    _close(got, ref.paged_attention(q, kv, tab, cl, cu, **kw), rtol=2e-2, atol=2e-2)
+    from mlxcel_b200.ops import _lib
+    assert _lib.read_status(torch.device(DEV)) == 0
+
+
 @pytest.mark.parametrize("tc", [True, False])
 @pytest.mark.parametrize("Hq,Hkv,D,window,sinks", [(8, 2, 128, 0, False), (4, 1, 64, 300, True), (4, 4, 128, 130, False)])
 def test_paged_prefill_long(monkeypatch, tc, Hq, Hkv, D, window, sinks):
