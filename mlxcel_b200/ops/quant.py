@@ -372,8 +372,10 @@ def qglu_linear(x: torch.Tensor, qt: QuantizedTensor, inter: int, act: str, bias
 
     M, K = x.shape
     if (x.is_cuda and M == 1 and _QMV_MAX_M >= 1 and qt.bits == 4 and qt.mode == "affine" and qt.packed.dim() == 2
-            and x.dtype == torch.bfloat16 and x.stride(1) == 1 and (bias is None or bias.dtype == torch.bfloat16)):
-        # one row: gate and up rows streamed once, activation in the epilogue (one launch)
+            and x.dtype == torch.bfloat16 and x.stride(1) == 1 and (bias is None or bias.dtype == torch.bfloat16)
+            and qt.packed.is_contiguous() and qt.scales.is_contiguous() and qt.biases.is_contiguous()):
+        # one row: gate and up rows streamed once, activation in the epilogue (one launch; rows are found by pointer, so strided
+        # parts are left to the form that re-tiles them)
         from . import _ACT_TO_EPI
         out = torch.empty(1, inter, dtype=torch.bfloat16, device=x.device)
         rc = _lib.load().mx_qmv_glu(x.data_ptr(), qt.packed.data_ptr(), qt.scales.data_ptr(), qt.biases.data_ptr(), out.data_ptr(),

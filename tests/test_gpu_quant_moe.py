@@ -97,6 +97,19 @@ def test_expert_streaming_shapes(monkeypatch, mode, group, counts, n_out, K, act
         _close(got[s], z, rtol=1e-2, atol=1e-2)
 
 
+def test_one_row_of_strided_weights():
+    """A gated projection of one row over a window of a wider packed matrix's columns: the rows do not lie back to back, so the
+    one-row kernel, which takes them by pointer, must leave the call to the form that re-tiles them."""
+    wide = _qt_to(quant.quantize(torch.randn(256, 512, generator=torch.Generator().manual_seed(3)) * 0.05, "affine", 4, 64), DEV)
+    parts = [wide.packed[:, 32:], wide.scales[:, 4:], wide.biases[:, 4:]]
+    x = torch.randn(1, 256, generator=torch.Generator().manual_seed(4)).to(torch.bfloat16).to(DEV)
+    want = quant.qglu_linear(x, quant.QuantizedTensor(*(t.contiguous() for t in parts), 4, 64, "affine"), 128, "silu")
+    for i in range(3):                                     # one strided part at a time, then all of them
+        some = [t if j == i else t.contiguous() for j, t in enumerate(parts)]
+        _close(quant.qglu_linear(x, quant.QuantizedTensor(*some, 4, 64, "affine"), 128, "silu"), want)
+    _close(quant.qglu_linear(x, quant.QuantizedTensor(*parts, 4, 64, "affine"), 128, "silu"), want)
+
+
 @pytest.mark.parametrize("mode,bits,group", [("affine", 4, 64), ("affine", 4, 128), ("affine", 8, 32), ("mxfp4", 4, 32)])
 @pytest.mark.parametrize("M", [1, 16, 64, 200])
 def test_fused_dequant_gemm(monkeypatch, mode, bits, group, M):
