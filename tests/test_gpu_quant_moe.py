@@ -110,6 +110,28 @@ def test_one_row_of_strided_weights():
     _close(quant.qglu_linear(x, quant.QuantizedTensor(*parts, 4, 64, "affine"), 128, "silu"), want)
 
 
+@pytest.mark.parametrize("mode,group,K", [("mxfp4", 32, 160), ("mxfp4", 32, 96), ("affine", 32, 160), ("affine", 64, 192)])
+@pytest.mark.parametrize("value", [float("nan"), float("inf")])
+def test_expert_streaming_keeps_rows_apart(mode, group, K, value):
+    """A weight row whose scales are not numbers spoils its own feature only. The last block of a row is not full there, so that
+    the words its scales are fetched by hold the next row's as well."""
+    E, n_out, rows = 3, 24, 5
+    g = torch.Generator().manual_seed(K)
+    qt = quant.quantize(torch.randn(E, n_out, K, generator=g) * 0.05, mode, 4, group)
+    if mode == "mxfp4":
+        qt.scales[:, 7] = 255
+    else:
+        qt.scales[:, 7], qt.biases[:, 7] = value, value
+    xs = torch.randn(rows, K, generator=g).to(torch.bfloat16)
+    off = torch.tensor([0, 2, 2, 5], dtype=torch.int32)
+    got = moe_ops.grouped_linear(xs.to(DEV), _qt_to(qt, DEV), off.to(DEV), n_out).cpu().float()
+    wd = quant.dequantize_ref(qt).float()
+    want = torch.cat([xs[off[e]:off[e + 1]].float() @ wd[e].t() for e in range(E)])
+    fine = torch.arange(n_out) != 7
+    assert not got[:, 7].isfinite().any() and got[:, fine].isfinite().all()
+    _close(got[:, fine], want[:, fine], rtol=1e-2, atol=1e-2)
+
+
 @pytest.mark.parametrize("mode,bits,group", [("affine", 4, 64), ("affine", 4, 128), ("affine", 8, 32), ("mxfp4", 4, 32)])
 @pytest.mark.parametrize("M", [1, 16, 64, 200])
 def test_fused_dequant_gemm(monkeypatch, mode, bits, group, M):
