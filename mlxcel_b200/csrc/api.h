@@ -331,6 +331,8 @@ int mx_qmv_glu(const void* x, const void* w, const void* scales, const void* bia
 // -9 = shape not covered (the caller falls back to the grouped GEMM).
 int mx_qstream(const void* xs, const void* w, const void* scales, const void* biases, const void* lin_bias, const int* offsets,
                void* out, int E, int rows_used, int n_out, int K, int group, int mode, int epi, float alpha, float limit, void* stream);
+// Whether that kernel asks for weights before it knows which experts have rows (1) or behind (0).
+int mx_qstream_ahead(int E, int rows_used);
 #ifdef __cplusplus
 }
 #endif

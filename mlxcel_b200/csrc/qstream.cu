@@ -6,7 +6,8 @@
 // is scarce, and everything is laid out around them (reference: gather_qmm for SwitchGLU, src/models/switch_layers.rs:98-220;
 // overlays/cuda/.../quantized/qmm/qmv.cu):
 //
-//   grid  = (K split, output-feature blocks, local experts); a block whose expert got no rows returns at once.
+//   grid  = (K split, output-feature blocks, local experts); a block whose expert got no rows returns as soon as it knows, and
+//           where few experts are in use nothing of its weights has been asked for by then (mx_qstream_ahead).
 //   warp  = one 16-row A tile of mma.sync m16n8k16: 16 features, or 8 features x (gate row, up row) when gated, so that a gate
 //           value and its up value meet in one lane. Every warp brings its own rows by cp.async into a ring of its own (64
 //           bytes = 128 weights of a row a stage, XOR-swizzled pieces), so no barrier stands between the stages.
@@ -22,7 +23,7 @@
 //
 // Measured on B200 (mxfp4, 128 experts of 2880 x 2880, top 4 of 128 rows): gate/up 393 us and down 211 us, 44 % of the copy
 // bandwidth; 1312 us for the two with the lanes of a quad reading the same 16 bytes and picking their codes by byte permutes.
-// 8 rows 127 and 75 us, 1 row 67 and 48 us. Issue slots and the latency between dependent instructions bound it.
+// 8 rows 97 and 56 us, 1 row 39 and 26 us. Issue slots and the latency between dependent instructions bound it.
 #include <cooperative_groups.h>
 #include <cuda_fp16.h>
 
@@ -48,6 +49,7 @@ struct QsParams {
   __nv_bfloat16* out;             // [rows, n_out]
   int N, K, n_out, epi;
   int k_per_cta;                  // multiple of 128
+  int ahead;                      // the first stages are loaded before it is known whether the expert has rows
   float alpha, limit;
 };
 
@@ -209,8 +211,10 @@ __global__ void __launch_bounds__(kQsThreads, QsShape<MODE, NT>::kResident) qstr
     ld_st = ld_st + S::kStageBytes == RING ? 0 : ld_st + S::kStageBytes;
     cp_async_commit();
   };
+  if (p.ahead) {                                                  // weights are nobody's output: before the wait
 #pragma unroll
-  for (int i = 0; i < S::kStages - 1; ++i) load();                // weights are nobody's output: before the wait
+    for (int i = 0; i < S::kStages - 1; ++i) load();
+  }
   pdl_wait();
   pdl_trigger();
 
@@ -218,6 +222,10 @@ __global__ void __launch_bounds__(kQsThreads, QsShape<MODE, NT>::kResident) qstr
   if (m_e <= 0) {                                                 // (the same for every CTA of the cluster)
     cp_async_wait<0>();
     return;
+  }
+  if (!p.ahead) {
+#pragma unroll
+    for (int i = 0; i < S::kStages - 1; ++i) load();
   }
   for (int t0 = 0; t0 < m_e; t0 += S::kTok) {
     const int toks = min(S::kTok, m_e - t0);
@@ -455,6 +463,13 @@ inline cudaError_t qs_dispatch(const QsParams& p, int E, int in_use, int rows_hi
 
 }  // namespace mx
 
+// Whether the first three stages are requested ahead of the dependent-launch wait, before the offsets can be read. An expert
+// without rows then has 3 of its stages read for nothing (3 of 23 for rows of 2880, twice that with K split in two), so this is
+// left to calls that expect rows nearly everywhere. Top 4 of 128 mxfp4 experts of 2880, gate/up and down (us), ahead / behind:
+// 1 row 62 and 46 / 39 and 26, 8 rows 115 and 69 / 97 and 56, 32 rows 250 and 134 / 246 and 131, 64 rows 333 and 176 / 333 and
+// 177, 128 rows 391 and 210 / 393 and 212; 128 affine experts of 768, groups of 32, 512 rows in all: 127 and 56 / 130 and 57.
+extern "C" int mx_qstream_ahead(int E, int rows_used) { return rows_used >= 2ll * E ? 1 : 0; }
+
 // xs [rows, K]; w [E, N, K/8] MLX-packed 4-bit (N = 2 * n_out rows, gate then up, when `epi` is a gated activation, else
 // N = n_out). mode: 0 affine (bf16 scales and biases per `group`), 1 mxfp4 (e8m0 scales per 32). offsets: device [E + 1] rows
 // of every expert. rows_used: how many rows are expected in all (any number is served; an expert with more than a pass holds
@@ -485,6 +500,7 @@ extern "C" int mx_qstream(const void* xs, const void* w, const void* scales, con
   p.out = static_cast<__nv_bfloat16*>(out);
   p.N = gated ? 2 * n_out : n_out, p.K = K, p.k_per_cta = 0;
   p.n_out = n_out, p.epi = epi, p.alpha = alpha, p.limit = limit;
+  p.ahead = mx_qstream_ahead(E, rows_used);
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   const int in_use = rows_used < E ? (rows_used > 0 ? rows_used : 1) : E;   // at most so many experts have rows
   const int hint = static_cast<int>(2ll * rows_used / E);   // (an expert's share varies: twice the average nearly always fits a pass)
