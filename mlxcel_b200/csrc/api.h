@@ -222,7 +222,7 @@ int mx_paged_prefill_tc(const void* q, long long q_stride, const void* k_pool, c
                         long long pool_blocks, const int* block_tables, const int* cu_q,
                         const int* context_lens, const float* sinks, void* out, int num_seqs,
                         int total_q, int max_q_len, int Hq, int Hkv, int D, int block_size,
-                        int max_blocks, int window, float scale, void* status, void* stream);
+                        int max_blocks, int window, float scale, int heads, void* status, void* stream);
 
 // Embedding gather: out[t, :] = table[ids[t], :] (bf16), ids outside [0, vocab) give zeros.
 int mx_embedding(const int* ids, const void* table, void* out, int T, int dim, int vocab,
@@ -333,6 +333,8 @@ int mx_qstream(const void* xs, const void* w, const void* scales, const void* bi
                void* out, int E, int rows_used, int n_out, int K, int group, int mode, int epi, float alpha, float limit, void* stream);
 // Whether that kernel asks for weights before it knows which experts have rows (1) or behind (0).
 int mx_qstream_ahead(int E, int rows_used);
+// Query heads a CTA of mx_paged_prefill_tc takes for these pieces: 1 or 2.
+int mx_prefill_heads(int num_seqs, int total_q, int max_q_len, int Hq, int Hkv);
 #ifdef __cplusplus
 }
 #endif

@@ -671,17 +671,31 @@ static int launch_prefill_tc(const CUtensorMap& mq, const CUtensorMap& mk, const
 
 using namespace mx;
 
+// Query heads a CTA of mx_paged_prefill_tc takes: two of a key head, where their number is even, unless the tiles of single heads
+// all find an SM of their own. Both forms take about as long for a tile pair as for a tile (us, contexts of 8192: heads of 128 138
+// for two, 128 for one; heads of 64 127 and 95), so two are better as soon as single heads need a second round of tiles (32 heads of
+// 128, one piece of 1024 tokens 144 against 250; 64 heads of 64, 512 tokens 129 against 186), and worse before (512 tokens 140
+// against 132; 64 heads of 64, 128 tokens 130 against 95; prompts of 128 tokens 12 against 10).
+extern "C" int mx_prefill_heads(int num_seqs, int total_q, int max_q_len, int Hq, int Hkv) {
+  if (Hq / Hkv % 2) return 1;
+  const long long by_length = static_cast<long long>(num_seqs) * ((max_q_len + kTcRows - 1) / kTcRows);
+  const long long by_tokens = total_q / kTcRows + static_cast<long long>(num_seqs);   // pieces of other lengths have fewer tiles
+  return (by_length < by_tokens ? by_length : by_tokens) * Hq > device_sm_count() ? 2 : 1;
+}
+
 // Tensor-core chunked prefill over a bf16 paged pool with 16-token blocks, D = 64 or 128.
 // Returns -10 when the configuration is not covered (the caller then uses mx_paged_prefill).
 // `q` rows are `q_stride` elements apart (16-byte aligned, q_stride % 8 == 0); `pool_blocks` is
-// the number of blocks in k_pool / v_pool; `status` is the device status word.
+// the number of blocks in k_pool / v_pool; `status` is the device status word. heads: query heads a CTA takes, 1 or 2, or 0 for
+// what mx_prefill_heads says.
 extern "C" int mx_paged_prefill_tc(const void* q, long long q_stride, const void* k_pool, const void* v_pool,
                                    long long pool_blocks, const int* block_tables, const int* cu_q,
                                    const int* context_lens, const float* sinks, void* out, int num_seqs,
                                    int total_q, int max_q_len, int Hq, int Hkv, int D, int block_size,
-                                   int max_blocks, int window, float scale, void* status, void* stream_) {
+                                   int max_blocks, int window, float scale, int heads, void* status, void* stream_) {
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   if (num_seqs <= 0 || total_q <= 0) return 0;
+  if (heads == 2 && Hkv > 0 && Hq / Hkv % 2) return -1;
   if (block_size != kTcBlock || (D != 64 && D != 128) || Hq % Hkv) return -10;
   if ((q_stride % 8) || (reinterpret_cast<uintptr_t>(q) & 15) || (reinterpret_cast<uintptr_t>(out) & 15))
     return -10;
@@ -711,8 +725,7 @@ extern "C" int mx_paged_prefill_tc(const void* q, long long q_stride, const void
   const uint64_t pool_rows = static_cast<uint64_t>(pool_blocks) * Hkv * kTcBlock;
   if (!make_tensor_map_bf16(&mk, k_pool, pool_rows, D, D, kTcBlock, 64)) return -4;
   if (!make_tensor_map_bf16(&mv, v_pool, pool_rows, D, D, kTcBlock, 64)) return -4;
-  if (Hq / Hkv % 2 == 0 && scale > 0.f) {
-    // two query heads of a key head per CTA; with an odd number of them (1 for plain multi-head attention) one
+  if (scale > 0.f && (heads != 0 ? heads : mx_prefill_heads(num_seqs, total_q, max_q_len, Hq, Hkv)) == 2) {
     PrefillTc2Params t{block_tables, cu_q, context_lens, sinks, p.out, p.status, num_seqs, Hq, Hkv, max_blocks, window, p.tiles_per_seq, p.scale_log2};
     return prefill_tc2_launch(mq, mk, mv, t, D, static_cast<int>(grid / 2), stream);
   }

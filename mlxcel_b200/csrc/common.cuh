@@ -376,6 +376,8 @@ inline cudaError_t launch_kernel(void (*kern)(KArgs...), dim3 grid, dim3 block, 
   return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
 }
 
+int device_sm_count();   // of the current device (gemm.cu)
+
 // Keep every kernel of the library on the same L1/shared-memory split (maximum shared): the
 // GEMM needs ~200 KB of shared memory per CTA, and alternating kernels that prefer different
 // splits makes the SM reconfigure between launches.

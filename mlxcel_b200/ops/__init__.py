@@ -278,6 +278,7 @@ def paged_decode(q: torch.Tensor, kv: KVLayer, block_tables: torch.Tensor,
 
 
 _PREFILL_TC = os.environ.get("MLXCEL_B200_PREFILL_TC", "1") != "0"
+_PREFILL_HEADS = 0      # query heads a CTA of the tcgen05 kernel takes: 0 = by the number of tiles (mx_prefill_heads); tests set 1 or 2
 # Pieces of at most this many 16-row tiles per sequence and key head go through the decode kernel with their tokens packed. It
 # reads the context once per tile (about 50 us a layer and tile at 16 x 4090 tokens, 8 key heads), the tcgen05 kernel once, but
 # with one CTA per (128-row tile, key head): 571 us there whatever the pieces hold.
@@ -325,7 +326,7 @@ def paged_prefill(q: torch.Tensor, kv: KVLayer, block_tables: torch.Tensor, cu_q
         rc = lib.mx_paged_prefill_tc(q.data_ptr(), q.stride(0), kv.k.data_ptr(), kv.v.data_ptr(), kv.k.shape[0],
                                      block_tables.data_ptr(), cu_q.data_ptr(), context_lens.data_ptr(),
                                      _lib.ptr(sinks), out.data_ptr(), S, T, max_q_len, Hq, Hkv, D, kv.block_size,
-                                     block_tables.shape[1], window, float(scale), ws.data_ptr(), _lib.stream())
+                                     block_tables.shape[1], window, float(scale), _PREFILL_HEADS, ws.data_ptr(), _lib.stream())
         if rc != -10:
             _lib.count_launch()
             _lib.check(rc, "mx_paged_prefill_tc")

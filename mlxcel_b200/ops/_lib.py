@@ -88,6 +88,7 @@ def _declare(lib) -> None:
         "mx_paged_verify": [_vp, _ll, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _f, _f,
                             _i, _i, _vp],
         "mx_qmv_glu": [_vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _f, _f, _vp],
+        "mx_prefill_heads": [_i, _i, _i, _i, _i],
         "mx_qstream_ahead": [_i, _i],
         "mx_qstream": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _f, _f, _vp],
         "mx_row_ssq": [_vp, _i, _i, _ll, _vp, _vp],
@@ -100,7 +101,7 @@ def _declare(lib) -> None:
         "mx_paged_prefill": [_vp, _ll, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i,
                              _i, _i, _i, _i, _i, _f, _f, _i, _vp],
         "mx_paged_prefill_tc": [_vp, _ll, _vp, _vp, _ll, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i,
-                                _i, _i, _i, _f, _vp, _vp],
+                                _i, _i, _i, _f, _i, _vp, _vp],
         "mx_embedding": [_vp, _vp, _vp, _i, _i, _i, _f, _vp],
         "mx_argmax": [_vp, _i, _ll, _vp, _i, _i, _vp],
         "mx_sample": [_vp, _i, _ll, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _vp],

@@ -350,9 +350,12 @@ def test_gemm_deferred_rmsnorm(M):
 @pytest.mark.parametrize("Hq,Hkv,D", [(2, 1, 128), (8, 2, 128), (4, 2, 64), (16, 1, 64), (6, 1, 128)])
 @pytest.mark.parametrize("ctx,qlen,window,sinks", [([128, 129, 700], [128, 129, 257], 0, False), ([1500, 127], [1000, 127], 0, True),
                                                    ([900, 300, 1], [300, 300, 1], 130, True), ([2300], [260], 1, False)])
-def test_paged_prefill_two_heads(Hq, Hkv, D, ctx, qlen, window, sinks):
-    """Two query heads of a key head per CTA: one key tile and many, tiles that end on an edge, behind it and inside a row, a single
-    row, windows of one key and across tiles, large logits that move the running maximum by more than the rescaling threshold."""
+@pytest.mark.parametrize("heads", [1, 2])
+def test_paged_prefill_two_heads(monkeypatch, heads, Hq, Hkv, D, ctx, qlen, window, sinks):
+    """Two query heads of a key head per CTA, and one, whatever the dispatch would take: one key tile and many, tiles that end on an
+    edge, behind it and inside a row, a single row, windows of one key and across tiles, large logits that move the running maximum
+    by more than the rescaling threshold."""
+    monkeypatch.setattr(ops, "_PREFILL_HEADS", heads)
     bs, nb = 16, 512
     kv = _pool(nb, Hkv, bs, D, 16)
     _fill_pool(kv, 7)
