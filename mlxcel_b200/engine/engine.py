@@ -635,6 +635,7 @@ class Engine:
                       num_prefill_seqs=sp, pf_block_tables=self.d_pf_tables[:sp] if sp else None,
                       pf_cu_q=self.d_cu[: sp + 1] if sp else None,
                       pf_context_lens=self.d_pf_lens[:sp] if sp else None, pf_max_q_len=max_q,
+                      pf_max_len=int(self.h_pf_lens[:sp].max()) if sp else 0,
                       pf_cu_q_host=cu if sp else None, logits_rows=self.d_rows[:R],
                       slot_mapping_win=self.d_slots_w[:t] if win else None,
                       dec_block_tables_win=self.d_dec_tables_w[:nd] if (win and nd) else None,

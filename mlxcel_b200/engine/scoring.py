@@ -33,7 +33,7 @@ def prefill_hidden(model, cfg, ids: list[int], block_size: int = 16) -> torch.Te
     i32 = dict(dtype=torch.int32, device=dev)
     b = StepBatch(token_ids=torch.tensor(ids, **i32), positions=torch.arange(T, **i32), slot_mapping=torch.arange(T, **i32),
                   num_prefill_seqs=1, pf_block_tables=torch.arange(nb, **i32)[None], pf_cu_q=torch.tensor([0, T], **i32),
-                  pf_context_lens=torch.tensor([T], **i32), pf_max_q_len=T, pf_cu_q_host=[0, T])
+                  pf_context_lens=torch.tensor([T], **i32), pf_max_q_len=T, pf_max_len=T, pf_cu_q_host=[0, T])
     b.seq_ids, b.pf_starts = [_SCRATCH_SEQ], [0]
     try:
         return model.forward_hidden(b, pool.layers)

@@ -45,6 +45,7 @@ class StepBatch:
     pf_cu_q: torch.Tensor | None = None            # [Sp+1] int32
     pf_context_lens: torch.Tensor | None = None    # [Sp] int32 (prefix + chunk)
     pf_max_q_len: int = 0
+    pf_max_len: int = 0                            # longest of pf_context_lens (0: not known on the host)
     pf_cu_q_host: list | None = None               # host copy of pf_cu_q (micro-batch splitting)
     logits_rows: torch.Tensor | None = None        # [R] int64 rows of the hidden state to project
     embeds: torch.Tensor | None = None             # optional [T, H] input embeddings (VLM / MTP)
@@ -295,7 +296,7 @@ class DecoderModel:
                 attn[:nd] = o
         if b.num_prefill_seqs > 0:
             o = ops.paged_prefill(q[nd:], kv, pf_tables, b.pf_cu_q, b.pf_context_lens,
-                                  max_q_len=b.pf_max_q_len, out=attn[nd:] if attn.is_cuda else None,
+                                  max_q_len=b.pf_max_q_len, max_len=b.pf_max_len, out=attn[nd:] if attn.is_cuda else None,
                                   **common)
             if not attn.is_cuda:
                 attn[nd:] = o

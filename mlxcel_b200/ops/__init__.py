@@ -6,6 +6,8 @@ PyTorch statements in :mod:`mlxcel_b200.ops.reference`, which are also the test 
 """
 from __future__ import annotations
 
+import functools
+import math
 import os
 
 from dataclasses import dataclass
@@ -279,17 +281,48 @@ def paged_decode(q: torch.Tensor, kv: KVLayer, block_tables: torch.Tensor,
 
 _PREFILL_TC = os.environ.get("MLXCEL_B200_PREFILL_TC", "1") != "0"
 _PREFILL_HEADS = 0      # query heads a CTA of the tcgen05 kernel takes: 0 = by the number of tiles (mx_prefill_heads); tests set 1 or 2
-# Pieces of at most this many 16-row tiles per sequence and key head go through the decode kernel with their tokens packed. It
-# reads the context once per tile (about 50 us a layer and tile at 16 x 4090 tokens, 8 key heads), the tcgen05 kernel once, but
-# with one CTA per (128-row tile, key head): 571 us there whatever the pieces hold.
+# Short pieces (verify rounds, short prompts) of at most this many 16-row tiles per sequence and key head may go through the decode
+# kernel with their tokens packed, see packed_splits.
 _VERIFY_TILES = 4
+
+
+@functools.lru_cache(maxsize=4096)
+def packed_splits(S: int, max_q: int, Hq: int, Hkv: int, D: int, keys: int, coded: bool, tc: bool) -> int:
+    """Splits of the keys with which pieces of at most ``max_q`` tokens on contexts of up to ``keys`` keys take the packed
+    form of the decode kernel, 0 where the kernels for longer pieces (``tc``: the tcgen05 one) are as fast or faster.
+
+    The packed form reads a context once per 16 rows of a key head and can split it, the others once per query head or pair of them
+    (tcgen05, 128 rows a CTA) or once per key head (8- and 4-bit pools), unsplit. Both sides are estimated as rounds of CTAs; the
+    constants (us) fit 588 calls of 1 to 24 pieces on 64 to 8192 keys to 9 % (heads of 128) and 12 % (64). Merging splits costs as
+    much as 1000 keys, so a split has 768 at least. In us, the other kernel against the packed form: 16 pieces of 4 tokens, 64 heads
+    over 8 of 128, 4096 keys 463 / 78; a single piece there 67 / 58; one of 16 tokens, 32 over 8 heads, 512 keys 13 / 17; 16
+    of 64 tokens, 32 heads over 32, 512 keys 52 / 126; the same over an 8-bit pool 225 / 179, on 64 keys 36 / 76."""
+    def rounds(ctas, slots):
+        x = ctas / slots
+        return 1.0 if x <= 1.0 else 0.5 * (x + math.ceil(x))
+    wide, G, sms = D == 128, Hq // Hkv, 148
+    t, whole = keys / 128, -(-keys // 128)                 # (tcgen05 tiles have 128 keys, the other kernels finish early)
+    if not tc:
+        other = rounds(S * Hkv * (-(-max_q * G // 128)), sms if wide else 1.5 * sms) * (4.5 + (12.9 if wide else 8.3) * t)
+    elif G % 2 == 0 and S * Hq > sms:
+        other = rounds(S * Hq // 2, sms) * ((7.5 + 2.2 * whole) if wide else (6.3 + 1.9 * whole))
+    else:
+        other = rounds(S * Hq, sms) * (6.5 + (1.95 if wide else 1.4) * whole)
+    pairs = S * Hkv * (-(-max_q // (16 // G)))
+    splits = max(1, min(2 * sms // pairs, keys // 768, 16))
+    slope = (4.0 if wide else 2.4) if coded else (2.0 if wide else 1.4)
+    packed = rounds(pairs * splits, 2 * sms) * ((10.0 if wide else 6.0) + slope * t / splits)
+    if splits > 1:
+        packed += (10.5 + 2.1 * splits) * (1.0 if wide else 0.6)
+    return splits if 1.1 * packed < other else 0
 
 
 def paged_prefill(q: torch.Tensor, kv: KVLayer, block_tables: torch.Tensor, cu_q: torch.Tensor,
                   context_lens: torch.Tensor, *, Hq: int, Hkv: int, D: int, scale: float,
                   max_q_len: int, window: int = 0, sinks: torch.Tensor | None = None,
-                  softcap: float = 0.0, out: torch.Tensor | None = None) -> torch.Tensor:
-    """Causal attention of query chunks against their sequences' paged KV (prefix + chunk)."""
+                  softcap: float = 0.0, out: torch.Tensor | None = None, max_len: int = 0) -> torch.Tensor:
+    """Causal attention of query chunks against their sequences' paged KV (prefix + chunk). ``max_len``: the longest of
+    ``context_lens`` where the caller knows it (0: what the block tables have room for); it only chooses between kernels."""
     T = q.shape[0]
     if not q.is_cuda:
         return ref.paged_attention(q, kv, block_tables, context_lens, cu_q, Hq=Hq, Hkv=Hkv, D=D,
@@ -300,26 +333,32 @@ def paged_prefill(q: torch.Tensor, kv: KVLayer, block_tables: torch.Tensor, cu_q
         return out
     S = context_lens.shape[0]
     G = Hq // Hkv
+    tc = (_PREFILL_TC and kv.kv_bits == 16 and kv.block_size == 16 and D in (64, 128) and softcap == 0.0
+          and kv.k.dtype == torch.bfloat16 and q.stride(0) % 8 == 0)
     # query tokens of a sequence that share a 16-row tile (for the calls that the kernels for longer pieces take too)
-    pack = 16 // G if G <= 16 and (G in (1, 2, 4, 8) or (_PREFILL_TC and kv.kv_bits == 16 and softcap == 0.0)) else 0
+    pack = 16 // G if G <= 16 and (G in (1, 2, 4, 8) or tc) else 0
+    splits = 0
     if pack and max_q_len <= _VERIFY_TILES * pack and kv.block_size == 16 and D in (64, 128) and q.stride(0) % 8 == 0 \
             and q.dtype == torch.bfloat16 and (kv.kv_bits != 16 or kv.k.dtype == torch.bfloat16):
-        # verify rounds: a few query tokens per sequence over long contexts
-        tiles = -(-max_q_len // pack)
-        splits = decode_splits(S * tiles, Hkv, block_tables.shape[1] * kv.block_size)
+        keys = max_len if max_len > 0 else block_tables.shape[1] * kv.block_size
+        if window > 0:
+            keys = min(keys, window + max_q_len)
+        splits = packed_splits(S, max_q_len, Hq, Hkv, D, -(-keys // 32) * 32, kv.kv_bits != 16, tc)
+    if splits:
         lib = _lib.load()
-        floats = int(lib.mx_paged_decode_scratch_floats(S * tiles, Hkv * pack * G, D, splits)) if splits > 1 else 0
-        scratch = _decode_scratch(q.device, floats)
+        scratch = None
+        if splits > 1:
+            tiles = -(-max_q_len // pack)
+            scratch = _decode_scratch(q.device, int(lib.mx_paged_decode_scratch_floats(S * tiles, Hkv * pack * G, D, splits)))
         rc = lib.mx_paged_verify(q.data_ptr(), q.stride(0), kv.k.data_ptr(), kv.v.data_ptr(), _lib.ptr(kv.k_meta), _lib.ptr(kv.v_meta),
                                  block_tables.data_ptr(), cu_q.data_ptr(), context_lens.data_ptr(), _lib.ptr(sinks), out.data_ptr(),
-                                 scratch.data_ptr(), S, max_q_len, Hq, Hkv, D, kv.block_size, block_tables.shape[1], window,
+                                 _lib.ptr(scratch), S, max_q_len, Hq, Hkv, D, kv.block_size, block_tables.shape[1], window,
                                  float(scale), float(softcap), kv.kv_bits, splits, _lib.stream())
         if rc != -10:
             _lib.count_launch()
             _lib.check(rc, "mx_paged_verify")
             return out
-    if (_PREFILL_TC and kv.kv_bits == 16 and kv.block_size == 16 and D in (64, 128) and softcap == 0.0
-            and kv.k.dtype == torch.bfloat16 and q.stride(0) % 8 == 0):
+    if tc:
         # tensor-core (tcgen05) kernel; -10 = configuration not covered, fall through
         lib = _lib.load()
         ws = _lib.workspace(q.device)

@@ -57,7 +57,7 @@ def split_batch(b: StepBatch, num_micro: int) -> list[tuple[StepBatch, slice]]:
                        pf_block_tables=b.pf_block_tables[s0:s1] if s1 > s0 else None,
                        pf_cu_q=(b.pf_cu_q[s0:s1 + 1] - cu[s0]).to(torch.int32) if s1 > s0 else None,
                        pf_context_lens=b.pf_context_lens[s0:s1] if s1 > s0 else None,
-                       pf_max_q_len=b.pf_max_q_len, pf_cu_q_host=[c - cu[s0] for c in cu[s0:s1 + 1]] if s1 > s0 else None)
+                       pf_max_q_len=b.pf_max_q_len, pf_max_len=b.pf_max_len, pf_cu_q_host=[c - cu[s0] for c in cu[s0:s1 + 1]] if s1 > s0 else None)
         out.append((mb, sel))
     return out
 

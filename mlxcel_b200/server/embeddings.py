@@ -26,7 +26,7 @@ def embed_texts(state, texts: list[str], pooling: str = "last") -> tuple[list[li
                       slot_mapping=torch.arange(T, dtype=torch.int32, device=dev), num_prefill_seqs=1,
                       pf_block_tables=torch.arange(nb, dtype=torch.int32, device=dev)[None],
                       pf_cu_q=torch.tensor([0, T], dtype=torch.int32, device=dev),
-                      pf_context_lens=torch.tensor([T], dtype=torch.int32, device=dev), pf_max_q_len=T)
+                      pf_context_lens=torch.tensor([T], dtype=torch.int32, device=dev), pf_max_q_len=T, pf_max_len=T)
         h = model.forward_hidden(b, pool.layers)
         if hasattr(model, "_norm"):          # the embedding is taken after the model's final norm
             h = model._norm(h, model.w.final_norm, model.w.extra.get("final_norm_b"))

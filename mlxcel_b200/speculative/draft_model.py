@@ -54,7 +54,7 @@ class DraftModelDrafter:
                       pf_block_tables=torch.from_numpy(tables).to(d),
                       pf_cu_q=torch.tensor(cu, dtype=torch.int32, device=d),
                       pf_context_lens=torch.tensor(lens, dtype=torch.int32, device=d),
-                      pf_max_q_len=max(len(t) for _, t, _ in items),
+                      pf_max_q_len=max(len(t) for _, t, _ in items), pf_max_len=max(lens),
                       logits_rows=torch.tensor([c - 1 for c in cu[1:]], device=d))
         return ops.argmax(self.model.forward(b, self.pool.layers)).cpu().tolist()
 

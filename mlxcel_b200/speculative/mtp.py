@@ -104,7 +104,7 @@ class MTPDrafter:
                       pf_block_tables=torch.from_numpy(tables).to(d),
                       pf_cu_q=torch.tensor(cu, dtype=torch.int32, device=d),
                       pf_context_lens=torch.tensor(lens, dtype=torch.int32, device=d),
-                      pf_max_q_len=max(len(t) for _, _, t, _ in items))
+                      pf_max_q_len=max(len(t) for _, _, t, _ in items), pf_max_len=max(lens))
         g = self.head.forward_hidden(b, self.pool.layers, hidden_in=x)
         rows = torch.tensor([c - 1 for c in cu[1:]], device=d)
         logits = self.head.logits(g, rows)

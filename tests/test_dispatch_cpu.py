@@ -1,6 +1,7 @@
 """The rules by which calls are sent to one kernel or another, as the kernel library and the bindings state them (no GPU needed)."""
 import pytest
 
+from mlxcel_b200 import ops
 from mlxcel_b200.ops import _lib
 
 
@@ -24,3 +25,27 @@ def test_expert_weights_are_asked_for_early_only_where_nearly_all_are_used(lib, 
 def test_prefill_takes_two_heads_where_single_ones_need_a_second_round(lib, seqs, tokens, longest, Hq, Hkv, heads):
     """148 SMs: tiles of 128 tokens times query heads, by the longest piece or, where pieces differ, by the tokens."""
     assert lib.mx_prefill_heads(seqs, tokens, longest, Hq, Hkv) == heads
+
+
+@pytest.mark.parametrize("S,max_q,Hq,Hkv,D,keys,coded,tc,packed", [
+    # many tiles: the context is read once per 16 rows, against once per 128 rows of one or two heads
+    (16, 64, 32, 32, 128, 64, False, True, False), (64, 64, 32, 32, 128, 512, False, True, False), (16, 48, 8, 8, 128, 4096, False, True, False),
+    (16, 64, 32, 32, 128, 64, True, False, False), (64, 8, 64, 8, 128, 64, True, False, False),
+    (64, 16, 32, 32, 128, 512, False, True, True), (16, 64, 32, 32, 128, 512, True, False, True),
+    # few tiles: either side is one round of CTAs, short contexts are over sooner without packing
+    (1, 16, 32, 8, 128, 16, False, True, False), (1, 4, 32, 8, 128, 512, False, True, False), (4, 4, 8, 8, 128, 512, False, True, False),
+    (1, 4, 32, 8, 128, 8192, False, True, True), (3, 4, 32, 8, 128, 12001, False, True, True), (1, 1, 16, 1, 128, 8192, False, True, True),
+    (1, 16, 32, 8, 128, 16, True, False, False), (1, 4, 32, 8, 128, 512, True, False, True),
+    # verify rounds
+    (16, 4, 64, 8, 128, 4096, False, True, True), (16, 4, 32, 8, 128, 4096, False, True, True), (8, 4, 64, 8, 64, 2048, False, True, True)])
+def test_short_pieces_are_packed_where_that_is_faster(S, max_q, Hq, Hkv, D, keys, coded, tc, packed):
+    """Calls that were timed on both sides (at least a tenth apart)."""
+    assert bool(ops.packed_splits(S, max_q, Hq, Hkv, D, keys, coded, tc)) == packed
+
+
+def test_key_splits_of_packed_pieces_follow_the_context():
+    """No split below 768 keys (merging costs as much as 1000), no more CTAs than two an SM, one split where the tiles fill the GPU."""
+    for S in (1, 3, 16, 64):
+        for keys in (128, 1024, 4096, 12032, 131072):
+            s = ops.packed_splits(S, 4, 32, 8, 128, keys, True, False)
+            assert s <= max(1, keys // 768) and s <= 16 and (s <= 1 or s * S * 8 <= 296)

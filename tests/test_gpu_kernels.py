@@ -273,6 +273,9 @@ def test_paged_prefill_short_pieces(monkeypatch, Hq, Hkv, D, bits, window, sinks
     (one sequence) and splits without keys."""
     if bits != 16 and Hq // Hkv not in (1, 2, 4, 8):
         pytest.skip("quantized pools are read for 1, 2, 4 or 8 query heads a key head")
+    # (the packed form whatever the dispatch would take; key splits as a decode step has them)
+    monkeypatch.setattr(ops, "packed_splits", lambda S, max_q, Hq, Hkv, D, keys, coded, tc: ops.decode_splits(
+        S * -(-max_q // (16 // (Hq // Hkv))), Hkv, keys))
     bs, nb = 16, 256
     kv = _pool(nb, Hkv, bs, D, bits)
     _fill_pool(kv, 6)
@@ -286,7 +289,7 @@ def test_paged_prefill_short_pieces(monkeypatch, Hq, Hkv, D, bits, window, sinks
     got = ops.paged_prefill(q, kv, tab, cu, cl, max_q_len=max(qlen), out=out, **kw)
     _close(got, ref.paged_attention(q, kv, tab, cl, cu, **kw), rtol=2e-2, atol=2e-2)
     # the kernels for longer pieces give the same
-    monkeypatch.setattr(ops, "_VERIFY_TILES", 0)
+    monkeypatch.setattr(ops, "packed_splits", lambda *a: 0)
     _close(got, ops.paged_prefill(q, kv, tab, cu, cl, max_q_len=max(qlen), **kw), rtol=2e-2, atol=2e-2)
 
 
