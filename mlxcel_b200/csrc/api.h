@@ -331,8 +331,9 @@ int mx_qmv_glu(const void* x, const void* w, const void* scales, const void* bia
 // -9 = shape not covered (the caller falls back to the grouped GEMM).
 int mx_qstream(const void* xs, const void* w, const void* scales, const void* biases, const void* lin_bias, const int* offsets,
                void* out, int E, int rows_used, int n_out, int K, int group, int mode, int epi, float alpha, float limit, void* stream);
-// Whether that kernel asks for weights before it knows which experts have rows (1) or behind (0).
-int mx_qstream_ahead(int E, int rows_used);
+// Whether that kernel asks for weights before it knows which experts have rows (1) or behind (0), with `ctas` blocks in all of
+// which `resident` are on the GPU at once.
+int mx_qstream_ahead(int E, int rows_used, long long ctas, int resident);
 // Query heads a CTA of mx_paged_prefill_tc takes for these pieces: 1 or 2.
 int mx_prefill_heads(int num_seqs, int total_q, int max_q_len, int Hq, int Hkv);
 #ifdef __cplusplus

@@ -413,7 +413,7 @@ __global__ void __launch_bounds__(kQsThreads, QsShape<MODE, NT>::kResident) qstr
 }
 
 template <int MODE, int NT, int LG>
-inline cudaError_t qs_launch(const QsParams& p, int E, int in_use, cudaStream_t stream) {
+inline cudaError_t qs_launch(const QsParams& p, int E, int in_use, int rows_used, cudaStream_t stream) {
   using S = QsShape<MODE, NT>;
   auto kern = qstream_kernel<MODE, NT, LG>;
   // function attributes are per device: a process that drives several GPUs sets them on each
@@ -438,6 +438,7 @@ inline cudaError_t qs_launch(const QsParams& p, int E, int in_use, cudaStream_t 
   while (splits < kQsMaxSplit && static_cast<long long>(blocks) * in_use * splits * 2 <= 256 && nblk / (splits * 2) >= 2) splits *= 2;
   a.k_per_cta = (nblk + splits - 1) / splits * kQsBlockK;
   splits = (p.K + a.k_per_cta - 1) / a.k_per_cta;
+  a.ahead = mx_qstream_ahead(E, rows_used, static_cast<long long>(splits) * blocks * E, S::kResident * device_sm_count());
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(splits, blocks, E);
   cfg.blockDim = dim3(kQsThreads);
@@ -455,20 +456,25 @@ inline cudaError_t qs_launch(const QsParams& p, int E, int in_use, cudaStream_t 
 }
 
 template <int MODE, int LG>
-inline cudaError_t qs_dispatch(const QsParams& p, int E, int in_use, int rows_hint, cudaStream_t stream) {
-  if (rows_hint <= 8) return qs_launch<MODE, 1, LG>(p, E, in_use, stream);
-  if (rows_hint <= 16) return qs_launch<MODE, 2, LG>(p, E, in_use, stream);
-  return qs_launch<MODE, 4, LG>(p, E, in_use, stream);
+inline cudaError_t qs_dispatch(const QsParams& p, int E, int rows_used, cudaStream_t stream) {
+  const int in_use = rows_used < E ? (rows_used > 0 ? rows_used : 1) : E;   // at most so many experts have rows
+  const int hint = static_cast<int>(2ll * rows_used / E);   // (an expert's share varies: twice the average nearly always fits a pass)
+  if (hint <= 8) return qs_launch<MODE, 1, LG>(p, E, in_use, rows_used, stream);
+  if (hint <= 16) return qs_launch<MODE, 2, LG>(p, E, in_use, rows_used, stream);
+  return qs_launch<MODE, 4, LG>(p, E, in_use, rows_used, stream);
 }
 
 }  // namespace mx
 
 // Whether the first three stages are requested ahead of the dependent-launch wait, before the offsets can be read. An expert
 // without rows then has 3 of its stages read for nothing (3 of 23 for rows of 2880, twice that with K split in two), so this is
-// left to calls that expect rows nearly everywhere. Top 4 of 128 mxfp4 experts of 2880, gate/up and down (us), ahead / behind:
+// left to calls that expect rows nearly everywhere, and to those whose blocks are all on the GPU at once (`ctas` of at most
+// `resident`), where the wait is what counts: 6 to 8 rows on 8 experts of 1408, 17 / 19. Top 4 of 128 mxfp4 experts of 2880, gate/up and down (us), ahead / behind:
 // 1 row 62 and 46 / 39 and 26, 8 rows 115 and 69 / 97 and 56, 32 rows 250 and 134 / 246 and 131, 64 rows 333 and 176 / 333 and
 // 177, 128 rows 391 and 210 / 393 and 212; 128 affine experts of 768, groups of 32, 512 rows in all: 127 and 56 / 130 and 57.
-extern "C" int mx_qstream_ahead(int E, int rows_used) { return rows_used >= 2ll * E ? 1 : 0; }
+extern "C" int mx_qstream_ahead(int E, int rows_used, long long ctas, int resident) {
+  return rows_used >= 2ll * E || ctas <= resident ? 1 : 0;
+}
 
 // xs [rows, K]; w [E, N, K/8] MLX-packed 4-bit (N = 2 * n_out rows, gate then up, when `epi` is a gated activation, else
 // N = n_out). mode: 0 affine (bf16 scales and biases per `group`), 1 mxfp4 (e8m0 scales per 32). offsets: device [E + 1] rows
@@ -500,12 +506,9 @@ extern "C" int mx_qstream(const void* xs, const void* w, const void* scales, con
   p.out = static_cast<__nv_bfloat16*>(out);
   p.N = gated ? 2 * n_out : n_out, p.K = K, p.k_per_cta = 0;
   p.n_out = n_out, p.epi = epi, p.alpha = alpha, p.limit = limit;
-  p.ahead = mx_qstream_ahead(E, rows_used);
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
-  const int in_use = rows_used < E ? (rows_used > 0 ? rows_used : 1) : E;   // at most so many experts have rows
-  const int hint = static_cast<int>(2ll * rows_used / E);   // (an expert's share varies: twice the average nearly always fits a pass)
-  if (mode == 1) return static_cast<int>(qs_dispatch<1, 5>(p, E, in_use, hint, stream));
-  if (group == 32) return static_cast<int>(qs_dispatch<0, 5>(p, E, in_use, hint, stream));
-  if (group == 64) return static_cast<int>(qs_dispatch<0, 6>(p, E, in_use, hint, stream));
-  return static_cast<int>(qs_dispatch<0, 7>(p, E, in_use, hint, stream));
+  if (mode == 1) return static_cast<int>(qs_dispatch<1, 5>(p, E, rows_used, stream));
+  if (group == 32) return static_cast<int>(qs_dispatch<0, 5>(p, E, rows_used, stream));
+  if (group == 64) return static_cast<int>(qs_dispatch<0, 6>(p, E, rows_used, stream));
+  return static_cast<int>(qs_dispatch<0, 7>(p, E, rows_used, stream));
 }

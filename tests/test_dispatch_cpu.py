@@ -12,10 +12,11 @@ def lib():
     return _lib.load()
 
 
-@pytest.mark.parametrize("experts,rows,ahead", [(128, 4, 0), (128, 128, 0), (128, 255, 0), (128, 256, 1), (8, 15, 0), (8, 16, 1), (1, 1, 0),
-                                                (1, 2, 1), (1 << 30, 1 << 30, 0)])
-def test_expert_weights_are_asked_for_early_only_where_nearly_all_are_used(lib, experts, rows, ahead):
-    assert lib.mx_qstream_ahead(experts, rows) == ahead
+@pytest.mark.parametrize("experts,rows,blocks,ahead", [(128, 4, 45, 0), (128, 128, 45, 0), (128, 255, 45, 0), (128, 256, 45, 1), (8, 15, 56, 0),
+                                                       (8, 16, 56, 1), (8, 6, 22, 1), (8, 2, 88, 0), (1, 1, 500, 0), (1 << 30, 1 << 30, 2, 0)])
+def test_expert_weights_are_asked_for_early_only_where_nearly_all_are_used(lib, experts, rows, blocks, ahead):
+    """... or where all blocks are on the GPU at once (444 of them)."""
+    assert lib.mx_qstream_ahead(experts, rows, experts * blocks, 444) == ahead
 
 
 @pytest.mark.parametrize("seqs,tokens,longest,Hq,Hkv,heads", [
