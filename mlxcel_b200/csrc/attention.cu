@@ -1181,14 +1181,8 @@ static int launch_decode_mma_bs(const DecodeParams& p, int G, int grid, cudaStre
   constexpr int smem = 16 * DK * 2 + ring;
   static_assert(ring >= kDmWarps * 16 * DV * 4, "merge buffer");
   auto kern = paged_decode_mma_kernel<DK, DV, KV_BITS, BS16, EXT, MEANS, PACK>;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return static_cast<int>(e);
-    cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
-                         cudaSharedmemCarveoutMaxShared);
-    configured = true;
-  }
+  static bool configured[64] = {};
+  if (const cudaError_t e = allow_shared(kern, smem, configured); e != cudaSuccess) return static_cast<int>(e);
   return static_cast<int>(launch_kernel(kern, dim3(grid), dim3(kDmThreads), smem, st, p, G));
 }
 
@@ -1226,13 +1220,8 @@ template <int D, int G, int KV_BITS>
 static int launch_prefill_one(const PrefillParams& p, int grid, cudaStream_t st) {
   constexpr int smem = (kPfRows + 4 * kPfKv) * D * 2;
   auto kern = paged_prefill_kernel<D, G, KV_BITS>;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return static_cast<int>(e);
-    prefer_max_shared(kern);
-    configured = true;
-  }
+  static bool configured[64] = {};
+  if (const cudaError_t e = allow_shared(kern, smem, configured); e != cudaSuccess) return static_cast<int>(e);
   kern<<<grid, kPfThreads, smem, st>>>(p);
   return static_cast<int>(cudaGetLastError());
 }

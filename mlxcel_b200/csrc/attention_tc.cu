@@ -657,13 +657,8 @@ static int launch_prefill_tc(const CUtensorMap& mq, const CUtensorMap& mk, const
                        (EXT ? 4 : 2) * SUB + 1024 + 256 + (EXT ? kExtSmem : 0);
   static_assert(smem <= 227 * 1024, "shared memory");
   auto kern = paged_prefill_tc_kernel<DK, DV, EXT, MAPS, MEANS>;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return static_cast<int>(e);
-    prefer_max_shared(kern);
-    configured = true;
-  }
+  static bool configured[64] = {};
+  if (const cudaError_t e = allow_shared(kern, smem, configured); e != cudaSuccess) return static_cast<int>(e);
   return static_cast<int>(launch_kernel(kern, dim3(grid), dim3(tc_threads(EXT)), smem, stream, mq, mk, mv, mkr, mvm, p));
 }
 

@@ -386,6 +386,19 @@ inline void prefer_max_shared(Kernel kern) {
   cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
                        cudaSharedmemCarveoutMaxShared);
 }
+// Allows a kernel `bytes` of dynamic shared memory, with the split above, the first time it is launched on the current device.
+// Function attributes are per device: `done` is the launcher's own flag for each, as a process may drive several GPUs.
+template <typename Kernel>
+inline cudaError_t allow_shared(Kernel kern, int bytes, bool (&done)[64]) {
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev >= 0 && dev < 64 && done[dev]) return cudaSuccess;
+  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (e != cudaSuccess) return e;
+  prefer_max_shared(kern);
+  if (dev >= 0 && dev < 64) done[dev] = true;
+  return cudaSuccess;
+}
 #define MX_PREFER_SHARED(kern)                                   \
   do {                                                           \
     static const bool mx_once_ = (::mx::prefer_max_shared(kern), true); \

@@ -398,13 +398,8 @@ __global__ void __launch_bounds__(256) latent_merge_kernel(const LatentDecodePar
 template <int MT>
 static int launch_latent_decode(const LatentDecodeParams& p, int grid, cudaStream_t st) {
   auto kern = latent_decode_kernel<MT>;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, ld_smem(kLdMaxRow, MT));
-    if (e != cudaSuccess) return static_cast<int>(e);
-    prefer_max_shared(kern);
-    configured = true;
-  }
+  static bool configured[64] = {};
+  if (const cudaError_t e = allow_shared(kern, ld_smem(kLdMaxRow, MT), configured); e != cudaSuccess) return static_cast<int>(e);
   return static_cast<int>(launch_kernel(kern, dim3(grid), dim3(kLdThreads), ld_smem(p.W, MT), st, p));
 }
 

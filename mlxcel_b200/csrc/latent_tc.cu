@@ -381,13 +381,8 @@ static int launch_latent_tc(const CUtensorMap& mq, const CUtensorMap& mp, Latent
   if (slots < np) return -10;
   t.slots = slots > 4 * np ? 4 * np : slots;
   auto kern = latent_decode_tc_kernel<N>;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, limit);
-    if (e != cudaSuccess) return static_cast<int>(e);
-    prefer_max_shared(kern);
-    configured = true;
-  }
+  static bool configured[64] = {};
+  if (const cudaError_t e = allow_shared(kern, limit, configured); e != cudaSuccess) return static_cast<int>(e);
   return static_cast<int>(launch_kernel(kern, dim3(grid), dim3(lt_threads(N)), fixed + t.slots * kLtSlot, st, mq, mp, t));
 }
 

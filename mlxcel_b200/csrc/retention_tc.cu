@@ -374,13 +374,8 @@ retention_chunk_kernel(const RetentionParams p, const float* __restrict__ cs, fl
 // scratch: cosines and sines of the angles [2, N, rot / 2]; o_raw: rows of the unnormed result [N, H, ret_vp(V)] where a head is wider than a tile.
 int launch_retention_chunks(const RetentionParams& p, float* scratch, float* o_raw, int pieces, int row0, int N, int* status, cudaStream_t st) {
   auto kern = retention_chunk_kernel;
-  static bool configured = false;
-  if (!configured) {
-    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kRtSmem);
-    if (e != cudaSuccess) return static_cast<int>(e);
-    prefer_max_shared(kern);
-    configured = true;
-  }
+  static bool configured[64] = {};
+  if (const cudaError_t e = allow_shared(kern, kRtSmem, configured); e != cudaSuccess) return static_cast<int>(e);
   const int half = p.rot / 2;
   if (half > 0) {
     const long long threads = static_cast<long long>(N) * half;

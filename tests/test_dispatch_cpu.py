@@ -1,4 +1,6 @@
 """The rules by which calls are sent to one kernel or another, as the kernel library and the bindings state them (no GPU needed)."""
+import re
+
 import pytest
 
 from mlxcel_b200 import ops
@@ -50,3 +52,12 @@ def test_key_splits_of_packed_pieces_follow_the_context():
         for keys in (128, 1024, 4096, 12032, 131072):
             s = ops.packed_splits(S, 4, 32, 8, 128, keys, True, False)
             assert s <= max(1, keys // 768) and s <= 16 and (s <= 1 or s * S * 8 <= 296)
+
+
+def test_shared_memory_is_allowed_on_every_device():
+    """Function attributes are per device: no launcher may keep one flag for all of them (a process that drives two GPUs would get a
+    launch error on the second)."""
+    for src in sorted((_lib.lib_path().parent.parent / "csrc").glob("*.cu")):
+        text = src.read_text()
+        if "MaxDynamicSharedMemorySize" in text or "allow_shared(" in text:
+            assert not re.search(r"static\s+bool\s+\w+\s*(=|;)", text), src.name
