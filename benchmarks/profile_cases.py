@@ -203,6 +203,7 @@ def gemm_graph(M=64, full=1):
 
     def graph_time(fn):
         s = torch.cuda.Stream()
+        s.wait_stream(torch.cuda.current_stream())        # (inputs are made there, in memory this stream must not write yet)
         with torch.cuda.stream(s):
             for _ in range(2):
                 fn()
@@ -305,6 +306,7 @@ def qgemm_graph():
 
     def graph_time(fn):
         s = torch.cuda.Stream()
+        s.wait_stream(torch.cuda.current_stream())        # (inputs are made there, in memory this stream must not write yet)
         with torch.cuda.stream(s):
             for _ in range(2):
                 fn()
@@ -469,6 +471,7 @@ def moe_decode(T=128, E=128, k=4, H=2880, inter=2880, reps=0):
 
     def graph_us(n=8):
         s = torch.cuda.Stream()
+        s.wait_stream(torch.cuda.current_stream())        # (inputs are made there, in memory this stream must not write yet)
         with torch.cuda.stream(s):
             for i in range(2):
                 run(i)

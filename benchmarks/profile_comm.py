@@ -116,6 +116,7 @@ def ep_main(rank: int, world: int, dev: torch.device) -> None:
             """The same 8 layers inside one CUDA graph (the epoch lives on the device, so a replay
             raises fresh flags)."""
             st = torch.cuda.Stream()
+            st.wait_stream(torch.cuda.current_stream())        # (inputs are made there, in memory this stream must not write yet)
             with torch.cuda.stream(st):
                 fn()
                 torch.cuda.synchronize()
@@ -177,6 +178,7 @@ def main() -> None:
 
     def graph_time(fn):
         s = torch.cuda.Stream()
+        s.wait_stream(torch.cuda.current_stream())        # (inputs are made there, in memory this stream must not write yet)
         with torch.cuda.stream(s):
             for _ in range(2):
                 fn()

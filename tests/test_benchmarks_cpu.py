@@ -53,3 +53,14 @@ def test_speculative_compare_harness_reports_lossless_runs():
                                     "--prompt-tokens", "24", "--max-tokens", "10", "--no-cuda-graphs"])
     assert row["same_tokens"] and row["classic_tok_s"] > 0 and row["speculative_tok_s"] > 0
     assert row["drafter"] == "prompt-lookup" and row["verify_rounds"] >= 0
+
+
+def test_side_streams_wait_for_the_stream_their_inputs_are_made_on():
+    """A benchmark that draws its inputs on the current stream and times on another one has to order the two: memory that the drawing
+    has given back may already be an output of the timed call."""
+    from pathlib import Path
+    for src in sorted(Path(__file__).parent.parent.joinpath("benchmarks").glob("*.py")):
+        lines = src.read_text().splitlines()
+        for line, then in zip(lines, lines[1:]):
+            if "= torch.cuda.Stream(" in line:
+                assert then.strip().startswith(line.split("=")[0].strip() + ".wait_stream("), (src.name, line)
