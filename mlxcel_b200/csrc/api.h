@@ -56,6 +56,9 @@ typedef struct MxGemmExtras {
   void* flags_mc;
   void* recv_mc;
   void* out_mc;
+  // Not 0 = `w` was written by work queued just before this call (weights expanded into a buffer). It is then read
+  // behind the dependent-launch wait like the other operands, not ahead of it like weights that nothing on the stream writes.
+  int w_fresh;
 } MxGemmExtras;
 
 // What a step of the fp32 residual stream adds besides a branch (NULL fields: nothing). In this order: the weighted sum of

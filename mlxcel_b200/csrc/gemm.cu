@@ -132,6 +132,7 @@ struct GemmParams {
   const float* ssq_in;  // consumer: every output row t is scaled by rsqrt(sum_p ssq / K_norm + eps)
   float* ssq_out;       // producer: per (feature tile, token) sum of squares of the bf16 results
   float ssq_eps, ssq_inv_dim;
+  int w_fresh;                  // no weight tile is requested ahead of the wait for the previous kernel
   int vec_ok;           // 16-byte vector epilogue allowed (N, strides and base addresses aligned)
   unsigned long long* trace;   // optional per-CTA phase timestamps (see MX_WS_TRACE_OFFSET)
   int l2_prefetch_kb;   // k-blocks of weights (beyond the smem ring) to prefetch into L2 before the wait
@@ -523,13 +524,14 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_lane,
     const uint64_t pol_x = l2_policy_evict_last();
     pol_lane = SWAP ? pol_w : pol_x;
     pol_col = SWAP ? pol_x : pol_w;
-    // Weights never depend on the previous kernel: the weight tiles of the first ring of stages
-    // are requested before waiting for it, so the weight stream of this GEMM starts while the
-    // previous kernel is still in its tail / epilogue. Activation tiles follow after the wait.
+    // Weights do not depend on the previous kernel (unless the call says so): the weight tiles of
+    // the first ring of stages are requested before waiting for it, so the weight stream of this
+    // GEMM starts while the previous kernel is still in its tail / epilogue. Activation tiles
+    // follow after the wait.
     if constexpr (!GROUPED) {
       GroupCursor c0;
       WorkItem it0;
-      if (decode_work<BN, SWAP, false>(p, blockIdx.x, c0, it0)) {
+      if (!p.w_fresh && decode_work<BN, SWAP, false>(p, blockIdx.x, c0, it0)) {
         const int kb0 = it0.split * p.kb_per_split;
         const int kb1 = min(p.num_kb, kb0 + p.kb_per_split);
         pre = min(p.stages, kb1 - kb0);
@@ -1875,6 +1877,8 @@ extern "C" int mx_gemm_bf16(const void* x, const void* w, void* out, const void*
   p.q_rows = w_rows;
   p.q_glu_tiles = glu ? glu_offset / kLaneRows : 0;
 
+  p.w_fresh = extras != nullptr && extras->w_fresh != 0;
+
   const int sms = device_sm_count();
   int bn;
   if (swap) {
@@ -1912,6 +1916,7 @@ extern "C" int mx_gemm_bf16(const void* x, const void* w, void* out, const void*
     pp.M = M, pp.N = N, pp.K = K, pp.ldo = ldo, pp.ldr = p.residual != nullptr ? ldr : 0;
     pp.glu_offset = glu_offset, pp.epilogue = epilogue, pp.glu_alpha = glu_alpha, pp.glu_limit = glu_limit;
     pp.ssq_in = p.ssq_in, pp.ssq_out = p.ssq_out, pp.ssq_eps = p.ssq_eps, pp.ssq_inv_dim = p.ssq_inv_dim;
+    pp.w_fresh = p.w_fresh;
     if (gemm_pair_wanted(pp, glu, sms)) {
       if (!make_tensor_map_bf16(&map_x, x, M, K, ldx, kLaneRows, kBK) ||
           !make_tensor_map_bf16(&map_w, w, w_rows, K, ldw, kLaneRows, kBK))
@@ -2040,6 +2045,7 @@ extern "C" int mx_gemm_comm(const void* x, const void* w, void* out, const void*
   p.comm.parity_stride = parity_stride;
   p.comm.rank_stride = rank_stride;
   if (const int rn = take_row_norm(p, extras, swap, N, mode); rn != 0) return rn;
+  p.w_fresh = extras != nullptr && extras->w_fresh != 0;
   if (extras != nullptr && extras->flags_mc != nullptr) {
     p.comm.nvls = 1;   // withdrawn in launch_gemm when the layout does not allow 16-byte multimem accesses
     p.comm.flags_mc = static_cast<uint32_t*>(extras->flags_mc);
@@ -2049,6 +2055,8 @@ extern "C" int mx_gemm_comm(const void* x, const void* w, void* out, const void*
   p.q_group = quant.group;
   p.q_groups_per_row = quant.wq != 0 ? K / quant.group : 0;
   p.q_rows = N;
+
+  p.w_fresh = extras != nullptr && extras->w_fresh != 0;
 
   const int sms = device_sm_count();
   int bn;

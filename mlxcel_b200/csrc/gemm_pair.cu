@@ -147,9 +147,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
       auto load_x = [&](int s, int kb, int m0) {
         gp_tma_load(ring + s * kGpStageBytes, &map_x, bars + 8 * s, kb * kGpBK, m0 + rank * 128, keep);
       };
-      // weights are nobody's output: the first ring of them is under way before the previous kernel has ended
+      // weights are nobody's output, unless the call says so: the first ring of them is under way before the previous kernel has ended
       int pre = 0;
-      if (pair < tiles) {
+      if (!p.w_fresh && pair < tiles) {
         int m0, f0;
         place(pair, m0, f0);
         pre = min(kGpStages, num_kb);

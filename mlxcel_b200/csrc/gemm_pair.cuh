@@ -17,6 +17,7 @@ struct GemmPairParams {
   const float* ssq_in;          // deferred RMSNorm, as in GemmParams
   float* ssq_out;
   float ssq_eps, ssq_inv_dim;
+  int w_fresh;
   int tiles_m, tiles_n, raster; // filled by the launch
 };
 

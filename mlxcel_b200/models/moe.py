@@ -28,8 +28,8 @@ def _dense(w):
 def _shared_expert(cfg, lw: LayerWeights, x: torch.Tensor) -> torch.Tensor:
     si = lw.shared_gate_up.shape[0] // 2 if not isinstance(lw.shared_gate_up, QuantizedTensor) \
         else lw.shared_gate_up.shape[-2] // 2
-    a = ops.glu_linear(x, _dense(lw.shared_gate_up), si, cfg.hidden_act)
-    s = ops.linear(a, _dense(lw.shared_down))
+    a = ops.glu_linear(x, _dense(lw.shared_gate_up), si, cfg.hidden_act, w_fresh=isinstance(lw.shared_gate_up, QuantizedTensor))
+    s = ops.linear(a, _dense(lw.shared_down), w_fresh=isinstance(lw.shared_down, QuantizedTensor))
     if lw.shared_gate is not None:
         g = torch.sigmoid(ops.linear(x, lw.shared_gate).float())
         s = (s.float() * g).to(s.dtype)

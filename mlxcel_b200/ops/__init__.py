@@ -78,12 +78,13 @@ def row_ssq(x: torch.Tensor, ssq: SsqBuffer) -> None:
 def linear(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None = None,
            residual: torch.Tensor | None = None, out: torch.Tensor | None = None,
            out_fp32: bool = False, force_mode: int = 0, force_splits: int = 0,
-           row_norm: "RowNorm | None" = None, ssq_out: "SsqBuffer | None" = None) -> torch.Tensor:
+           row_norm: "RowNorm | None" = None, ssq_out: "SsqBuffer | None" = None, w_fresh: bool = False) -> torch.Tensor:
     """``x[M,K] @ w[N,K]^T (+ bias) (+ residual)`` with bf16 operands, fp32 accumulation.
 
     ``row_norm``: deferred RMSNorm — ``x`` is un-normalised, the norm weight is folded into ``w`` and
     every output row is scaled by the 1/rms described by ``row_norm.ssq`` before the bias.
-    ``ssq_out``: the kernel also leaves the per-tile sums of squares of its result rows there."""
+    ``ssq_out``: the kernel also leaves the per-tile sums of squares of its result rows there.
+    ``w_fresh``: ``w`` was written by a kernel queued just before (the GEMM otherwise asks for weights ahead of its turn)."""
     if not x.is_cuda:
         assert row_norm is None and ssq_out is None, "deferred RMSNorm is a CUDA-only path"
         return ref.linear(x, w, bias, residual, torch.float32 if out_fp32 else None)
@@ -100,7 +101,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None = None,
         return out
     epi = EPI_RESIDUAL if residual is not None else (EPI_BIAS if bias is not None else EPI_NONE)
     ws = _lib.workspace(x.device)
-    ex = _lib.gemm_extras(row_norm=row_norm, ssq_out=ssq_out)
+    ex = _lib.gemm_extras(row_norm=row_norm, ssq_out=ssq_out, w_fresh=w_fresh)
     _lib_call("mx_gemm_bf16", x.data_ptr(), w.data_ptr(), out.data_ptr(), _lib.ptr(bias),
               _lib.ptr(residual), M, N, K, x.stride(0), w.stride(0), out.stride(0),
               residual.stride(0) if residual is not None else 0, epi, 1 if out_fp32 else 0, 0,
@@ -127,7 +128,7 @@ def _linear_any(x, w, bias, residual, out, out_fp32: bool) -> torch.Tensor:
 def glu_linear(x: torch.Tensor, w: torch.Tensor, inter: int, act: str = "silu",
                bias: torch.Tensor | None = None, alpha: float = 1.702, limit: float = 7.0,
                out: torch.Tensor | None = None, force_mode: int = 0,
-               force_splits: int = 0, row_norm: "RowNorm | None" = None) -> torch.Tensor:
+               force_splits: int = 0, row_norm: "RowNorm | None" = None, w_fresh: bool = False) -> torch.Tensor:
     """``act(x @ w[:I]^T) * (x @ w[I:2I]^T)`` — gate/up projection with the activation fused
     into the GEMM epilogue (gate and up live in two TMEM accumulators)."""
     epi = _ACT_TO_EPI[act]
@@ -137,13 +138,13 @@ def glu_linear(x: torch.Tensor, w: torch.Tensor, inter: int, act: str = "silu",
     assert w.shape[0] == 2 * inter and x.stride(1) == 1 and w.stride(1) == 1
     if x.dtype == torch.float32 or inter % 8 or K % 8 or x.stride(0) % 8 or w.stride(0) % 8 or (x.data_ptr() | w.data_ptr()) % 16:
         assert row_norm is None and bias is None, "this form has no bias and no deferred RMSNorm"
-        return _glu_any(x, w, inter, epi, alpha, limit, out)
+        return _glu_any(x, w, inter, epi, alpha, limit, out, w_fresh)
     if out is None:
         out = torch.empty(M, inter, dtype=torch.bfloat16, device=x.device)
     if M == 0:
         return out
     ws = _lib.workspace(x.device)
-    ex = _lib.gemm_extras(row_norm=row_norm)
+    ex = _lib.gemm_extras(row_norm=row_norm, w_fresh=w_fresh)
     _lib_call("mx_gemm_bf16", x.data_ptr(), w.data_ptr(), out.data_ptr(), _lib.ptr(bias), None, M,
               inter, K, x.stride(0), w.stride(0), out.stride(0), 0, epi, 0, inter, float(alpha),
               float(limit), ws.data_ptr(), ws.numel(), force_mode, force_splits, _lib.stream(),
@@ -151,9 +152,9 @@ def glu_linear(x: torch.Tensor, w: torch.Tensor, inter: int, act: str = "silu",
     return out
 
 
-def _glu_any(x, w, inter: int, epi: int, alpha: float, limit: float, out) -> torch.Tensor:
+def _glu_any(x, w, inter: int, epi: int, alpha: float, limit: float, out, w_fresh: bool = False) -> torch.Tensor:
     """:func:`glu_linear` as projection and activation kernel, for fp32 operands and sizes the fused form does not take."""
-    z = linear(x, w)
+    z = linear(x, w, w_fresh=w_fresh)
     out = torch.empty(x.shape[0], inter, dtype=x.dtype, device=x.device) if out is None else out
     if x.shape[0]:
         _lib_call("mx_glu_rows", z.data_ptr(), z.stride(0), out.data_ptr(), x.shape[0], inter, epi, float(alpha), float(limit),

@@ -147,20 +147,20 @@ def _declare(lib) -> None:
 
 class GemmExtras(ctypes.Structure):
     """Mirror of ``MxGemmExtras`` (csrc/api.h): the optional per-call arguments of the GEMM entry
-    points — packed-weight format, deferred-RMSNorm buffers, NVLS multicast addresses."""
+    points — packed-weight format, deferred-RMSNorm buffers, NVLS multicast addresses, weights written just before."""
 
     _fields_ = [("wq", _i), ("q_group", _i), ("ssq_in", _vp), ("ssq_out", _vp), ("ssq_eps", _f),
-                ("ssq_inv_dim", _f), ("flags_mc", _vp), ("recv_mc", _vp), ("out_mc", _vp)]
+                ("ssq_inv_dim", _f), ("flags_mc", _vp), ("recv_mc", _vp), ("out_mc", _vp), ("w_fresh", _i)]
 
 
 def gemm_extras(wq: int = 0, q_group: int = 0, row_norm=None, ssq_out=None, flags_mc: int = 0,
-                recv_mc: int = 0, out_mc: int = 0):
+                recv_mc: int = 0, out_mc: int = 0, w_fresh: bool = False):
     """Builds the extras argument of one GEMM call (``None`` when the call needs none). The returned
     object must stay referenced until the call returns (pass ``ctypes.byref`` of it)."""
-    if not (wq or row_norm is not None or ssq_out is not None or flags_mc):
+    if not (wq or row_norm is not None or ssq_out is not None or flags_mc or w_fresh):
         return None
     ex = GemmExtras()
-    ex.wq, ex.q_group = int(wq), int(q_group)
+    ex.wq, ex.q_group, ex.w_fresh = int(wq), int(q_group), int(w_fresh)
     if row_norm is not None:
         ex.ssq_in = row_norm.ssq.buf.data_ptr()
         ex.ssq_eps = float(row_norm.eps)

@@ -336,8 +336,9 @@ def tile_experts_for_gemm(qt: QuantizedTensor, glu_inter: int | None = None) -> 
 
 def quant_extras(qt: QuantizedTensor, wq: int, **kw):
     """(pointer to the re-tiled packed weights, extras describing them) for one GEMM call."""
+    fresh = getattr(qt, "_gemm_tiles", None) is None           # (written by the kernels queued just before)
     tiles = tile_for_gemm(qt)
-    return tiles.data_ptr(), _lib.gemm_extras(wq=wq, q_group=qt.group_size, **kw)
+    return tiles.data_ptr(), _lib.gemm_extras(wq=wq, q_group=qt.group_size, w_fresh=fresh, **kw)
 
 
 def _fused_qgemm(x, qt, wq, out, bias, residual, inter=None, act=None, alpha=1.702, limit=7.0):
@@ -425,4 +426,4 @@ def qlinear(x: torch.Tensor, qt: QuantizedTensor, bias=None, residual=None, out=
         tmp = torch.empty(N, K, dtype=torch.bfloat16, device=x.device)
         _TMP[key] = tmp
     dequantize(qt, tmp)
-    return linear(x, tmp, bias=bias, residual=residual, out=out)
+    return linear(x, tmp, bias=bias, residual=residual, out=out, w_fresh=True)

@@ -1,10 +1,13 @@
 """The rules by which calls are sent to one kernel or another, as the kernel library and the bindings state them (no GPU needed)."""
 import re
+from types import SimpleNamespace
 
 import pytest
+import torch
 
 from mlxcel_b200 import ops
-from mlxcel_b200.ops import _lib
+from mlxcel_b200.models import moe
+from mlxcel_b200.ops import _lib, quant
 
 
 @pytest.fixture(scope="module")
@@ -61,3 +64,23 @@ def test_shared_memory_is_allowed_on_every_device():
         text = src.read_text()
         if "MaxDynamicSharedMemorySize" in text or "allow_shared(" in text:
             assert not re.search(r"static\s+bool\s+\w+\s*(=|;)", text), src.name
+
+
+def test_expanded_weights_are_not_read_ahead(monkeypatch):
+    """A GEMM asks for its first weights before the kernel ahead of it has ended. Where that kernel expands the weights into a buffer the
+    call has to say so: nothing else orders the two."""
+    seen = []
+    monkeypatch.setattr(ops, "linear", lambda x, w, **kw: seen.append(kw.get("w_fresh", False)))
+    monkeypatch.setattr(ops, "glu_linear", lambda x, w, *a, **kw: seen.append(kw.get("w_fresh", False)))
+    monkeypatch.setattr(quant, "dequantize", lambda qt, out=None: out)
+    monkeypatch.setattr(quant, "_TMP", {})
+    monkeypatch.setattr(_lib, "load", lambda: None)
+    packed, dense = quant.quantize(torch.randn(32, 64), "affine", 4, 64), torch.randn(32, 64)
+    x = SimpleNamespace(is_cuda=True, shape=(300, 64), device=torch.device("cpu"))
+    quant.qlinear(x, packed)
+    for w in (packed, dense):
+        moe._shared_expert(SimpleNamespace(hidden_act="silu"), SimpleNamespace(shared_gate_up=w, shared_down=w, shared_gate=None), x)
+    assert seen == [True, True, True, False, False]
+    # the re-tiled copy of packed weights: built by the first call
+    assert [quant.quant_extras(packed, 1)[1].w_fresh for _ in range(2)] == [1, 0]
+    assert _lib.gemm_extras(w_fresh=True).w_fresh == 1 and _lib.gemm_extras() is None
