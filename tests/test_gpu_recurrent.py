@@ -128,6 +128,28 @@ def test_ssm_scan_varlen(H, P, N, G, n_short):
     _close(st.cpu(), st2, rtol=2e-3, atol=2e-3)
 
 
+@pytest.mark.parametrize("shift", [0, 1, 4])
+@pytest.mark.parametrize("H,P,N,G", [(4, 64, 128, 2), (3, 40, 64, 1), (8, 32, 32, 1), (2, 8, 16, 2)])
+def test_ssm_scan_tails(H, P, N, G, shift):
+    """Row kernel: pieces that end one, two and three steps into a group of four and at the ends of chunks; B and C that 16-byte
+    accesses can and cannot reach (odd columns, rows of an odd number of elements)."""
+    lens = [2, 3, 5, 18, 16, 33, 7]
+    cu, slots, reset = _ragged(lens, 7)
+    T, wide = int(cu[-1]), H * P + 2 * G * N
+    conv = _bf(T, wide + (8 if shift == 0 else 5), sc=0.5)[:, shift:shift + wide]
+    x, Bm, Cm = conv[:, :H * P], conv[:, H * P:H * P + G * N], conv[:, H * P + G * N:]
+    dt = _bf(T, H)
+    A = -torch.rand(H, device=DEV) - 0.1
+    D, db = torch.randn(H, device=DEV), torch.randn(H, device=DEV) * 0.1
+    st = torch.randn(7, H, P, N, device=DEV) * 0.2
+    st2 = st.clone().cpu()
+    y = R.ssm_scan_varlen(st, slots.to(DEV), cu.to(DEV), reset.to(DEV), x, dt, A, Bm, Cm, D, db, True, (0.01, 0.8), 0)
+    yr = R.ssm_scan_varlen_ref(st2, slots, cu, reset, x.cpu(), dt.cpu(), A.cpu(), Bm.cpu(), Cm.cpu(), D.cpu(), db.cpu(), True, (0.01, 0.8))
+    # y: one rounding to bf16 (2^-8) and fp32 sums of N products; the state: fp32, a few operations a step and exp(dt A) to 2 ulp
+    assert ((y.cpu().float() - yr.float()).abs() <= yr.float().abs() * 2 ** -7 + 1e-3).all()
+    assert ((st.cpu() - st2).abs() <= st2.abs() * 1e-4 + 1e-4).all()
+
+
 @pytest.mark.parametrize("dim,groups,off", [(640, 1, 40), (640, 5, 40), (644, 2, 3), (8192, 1, 0)])
 def test_gated_rmsnorm(dim, groups, off):
     y, full = _bf(77, dim), _bf(77, dim + 360)
