@@ -339,6 +339,8 @@ int mx_qstream(const void* xs, const void* w, const void* scales, const void* bi
 int mx_qstream_ahead(int E, int rows_used, long long ctas, int resident);
 // Query heads a CTA of mx_paged_prefill_tc takes for these pieces: 1 or 2.
 int mx_prefill_heads(int num_seqs, int total_q, int max_q_len, int Hq, int Hkv);
+// Whether mx_gemm_bf16 takes a call of so many rows and (gated) features on pairs of SMs, if strides and addresses allow: 1 or 0.
+int mx_gemm_on_pairs(int M, int N, int glu);
 #ifdef __cplusplus
 }
 #endif

@@ -308,13 +308,16 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
 // tiles takes at least 1.25 times a wave of pair tiles (5 waves against 4 at M 543, N 28672: 143 us against 154; 4 against 3 at M
 // 300: 118 against 118); gated it takes about as long (8192 x 14336, K 4096: 1575 against 1644; 5 against 4 waves at M 543: 155
 // against 134), as the single-SM kernel's gated epilogue has half the outputs to write.
+static bool pair_is_faster(int M, int N, bool glu, int sms) {
+  if (M <= 256 || (!glu && N <= 128)) return false;
+  const int feats = glu ? 128 : 256;
+  const long long n = (N + feats - 1) / feats, pairs = sms / 2;
+  const long long waves = ((M + 255) / 256 * n + pairs - 1) / pairs, single = ((M + 127) / 128 * n + sms - 1) / sms;
+  return waves * 100 <= single * (glu ? 104 : 125);
+}
 bool gemm_pair_wanted(const GemmPairParams& p, bool glu, int sms) {
   const uintptr_t a = reinterpret_cast<uintptr_t>(p.out) | reinterpret_cast<uintptr_t>(p.residual);
-  if (p.M <= 256 || p.N % 8 || p.ldo % 8 || p.ldr % 8 || (a & 15) || p.status == nullptr || (!glu && p.N <= 128)) return false;
-  const int feats = glu ? 128 : 256;
-  const long long n = (p.N + feats - 1) / feats, pairs = sms / 2;
-  const long long waves = ((p.M + 255) / 256 * n + pairs - 1) / pairs, single = ((p.M + 127) / 128 * n + sms - 1) / sms;
-  return waves * 100 <= single * (glu ? 104 : 125);
+  return p.N % 8 == 0 && p.ldo % 8 == 0 && p.ldr % 8 == 0 && (a & 15) == 0 && p.status != nullptr && pair_is_faster(p.M, p.N, glu, sms);
 }
 
 int gemm_pair_launch(const CUtensorMap& map_x, const CUtensorMap& map_w, GemmPairParams p, bool glu, int sms, cudaStream_t stream) {
@@ -340,3 +343,5 @@ int gemm_pair_launch(const CUtensorMap& map_x, const CUtensorMap& map_w, GemmPai
 }
 
 }  // namespace mx
+
+extern "C" int mx_gemm_on_pairs(int M, int N, int glu) { return N % 8 == 0 && mx::pair_is_faster(M, N, glu != 0, mx::device_sm_count()); }

@@ -89,6 +89,7 @@ def _declare(lib) -> None:
                             _i, _i, _vp],
         "mx_qmv_glu": [_vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _f, _f, _vp],
         "mx_prefill_heads": [_i, _i, _i, _i, _i],
+        "mx_gemm_on_pairs": [_i, _i, _i],
         "mx_qstream_ahead": [_i, _i, _ll, _i],
         "mx_qstream": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _f, _f, _vp],
         "mx_row_ssq": [_vp, _i, _i, _ll, _vp, _vp],

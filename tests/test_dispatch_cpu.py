@@ -84,3 +84,11 @@ def test_expanded_weights_are_not_read_ahead(monkeypatch):
     # the re-tiled copy of packed weights: built by the first call
     assert [quant.quant_extras(packed, 1)[1].w_fresh for _ in range(2)] == [1, 0]
     assert _lib.gemm_extras(w_fresh=True).w_fresh == 1 and _lib.gemm_extras() is None
+
+
+@pytest.mark.parametrize("M,N,glu,pairs", [(256, 4096, 0, 0), (257, 264, 0, 1), (257, 264, 1, 1), (512, 128, 0, 0), (512, 136, 0, 1), (600, 136, 0, 1),
+                                           (300, 28672, 0, 0), (543, 28672, 0, 1), (543, 14336, 1, 0), (2048, 14336, 1, 1), (8192, 4096, 0, 1),
+                                           (512, 4100, 0, 0)])
+def test_gemms_on_pairs_of_sms(lib, M, N, glu, pairs):
+    """More than 256 rows, features in 16-byte pieces, and no last wave of tiles that costs more than the pairing gives."""
+    assert lib.mx_gemm_on_pairs(M, N, glu) == pairs

@@ -9,8 +9,9 @@ DEV = "cuda"
 
 
 def _close(got, want, rtol=2e-2, atol=2e-2):
-    err = (got.float() - want.float()).abs()
-    bad = (err > atol + rtol * want.float().abs()).sum().item()
+    got, want = got.float(), want.float()
+    err = (got - want).abs()
+    bad = (~((err <= atol + rtol * want.abs()) | (got == want))).sum().item()          # (a NaN is no match)
     assert bad == 0, f"{bad}/{err.numel()} mismatches, max err {err.max().item():.4g}"
 
 
