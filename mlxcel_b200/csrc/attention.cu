@@ -635,8 +635,9 @@ constexpr int kDmKeys = 16;  // keys per group (one MMA k-step of P V)
 //
 // PACK: verify rounds. A sequence has a few query tokens instead of one; as many of them as fit make the tile's 16 rows (row =
 // token * heads per key + head), each with its own causal limit, so that the context is read once per 16 / heads tokens. 16
-// sequences x 4 tokens on contexts of about 4000, 64 query and 8 key heads of 128: 571 us a layer with the tcgen05 prompt kernel
-// (128 rows a tile, 32 of them used, one CTA for a whole context), the whole step of 3 layers 2304 us before, 1276 us with this.
+// sequences x 4 tokens on contexts of 4096, 64 query and 8 key heads of 128: 463 us a layer with the tcgen05 prompt kernel (one query
+// head a CTA, 4 of its 128 rows used, a whole context each; 283 us in its two-head form), 79 us with this. Where it is taken and
+// with how many splits: packed_splits in the bindings.
 template <int DK, int DV, int KV_BITS, bool BS16, bool EXT, bool MEANS, bool PACK = false>
 __global__ void __launch_bounds__(kDmThreads)
 paged_decode_mma_kernel(const DecodeParams p, const int heads_per_key) {

@@ -335,9 +335,11 @@ __device__ __forceinline__ void dequant_half_row_to_tile(const uint8_t* pk_row, 
   if constexpr (WQ == 1) {
     // affine 4-bit on packed bf16 pairs: (w >> 4i) & 0x000F000F | 0x43004300 is the bf16 pair (128 + n_2i, 128 + n_2i+1) -
     // the re-tiled words hold the codes in that order -, minus 128 is exact, then one fused multiply-add per pair (q * scale +
-    // bias, rounded once to bf16). The integer pipe is the busiest: with the codes in checkpoint order four byte permutes more a
-    // word, 32 rows took 47.5 us on 28672 x 4096 gated (45.0 so) and 206 us on 128256 x 4096 (196). Neither more unpacking warps,
-    // in groups that take k-blocks in turn, nor deeper rings of packed blocks made it faster.
+    // bias, rounded once to bf16). No pipe is full (32 rows, 28672 x 4096 gated: integer 39 %, issue slots 39 %, DRAM 19 %; a warp
+    // that could issue waits for a load or a barrier 2.1 and for a fixed latency 1.3 times as long as it issues): what bounds it is
+    // the chain of a stage, packed block, shared load, conversion, store, fence, arrival. Each instruction taken out of it counts:
+    // with the codes in checkpoint order four byte permutes more a word, 32 rows took 47.5 us on 28672 x 4096 gated (45.0 so) and
+    // 206 us on 128256 x 4096 (196). Neither more unpacking warps, in groups that take k-blocks in turn, nor deeper rings helped.
     const uint4 v = *reinterpret_cast<const uint4*>(pk_row + half * 16);
     const uint32_t wds[4] = {v.x, v.y, v.z, v.w};
     const __nv_bfloat162 s2 = __halves2bfloat162(sb, sb), b2 = __halves2bfloat162(bb, bb);

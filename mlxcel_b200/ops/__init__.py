@@ -295,9 +295,9 @@ def packed_splits(S: int, max_q: int, Hq: int, Hkv: int, D: int, keys: int, code
     The packed form reads a context once per 16 rows of a key head and can split it, the others once per query head or pair of them
     (tcgen05, 128 rows a CTA) or once per key head (8- and 4-bit pools), unsplit. Both sides are estimated as rounds of CTAs; the
     constants (us) fit 588 calls of 1 to 24 pieces on 64 to 8192 keys to 9 % (heads of 128) and 12 % (64). Merging splits costs as
-    much as 1000 keys, so a split has 768 at least. In us, the single-head or 8-bit kernel against the packed form: 16 pieces of 4 tokens, 64 heads
-    over 8 of 128, 4096 keys 463 / 79; one such piece 67 / 44; one of 64 tokens, 32 heads over 32, 1024 keys 21 / 25; 16 of them on
-    512 keys 52 / 126; the same over an 8-bit pool 225 / 180, on 64 keys 36 / 76."""
+    much as 1000 keys, so a split has 768 at least. In us, the single-head or 8-bit kernel against the packed form: 16 pieces of 4
+    tokens, 64 heads over 8 of 128, 4096 keys 463 / 79; one such piece 67 / 44; one of 64 tokens, 32 heads over 32, 1024 keys
+    21 / 25; 16 of them on 512 keys 52 / 126; the same over an 8-bit pool 225 / 180, on 64 keys 36 / 76."""
     def rounds(ctas, slots):
         x = ctas / slots
         return 1.0 if x <= 1.0 else 0.5 * (x + math.ceil(x))

@@ -121,11 +121,13 @@ def route(logits: torch.Tensor, k: int, mode: str = "topk_softmax", norm_topk: b
 
 
 _QGEMV_MAX_ROWS = int(os.environ.get("MLXCEL_B200_MOE_QGEMV_MAX_ROWS", "16"))
-# From this many rows per expert (on average) packed 4-bit experts are expanded to bf16 once and run
-# through the dense grouped GEMM: the expansion is one pass over the layer's experts at memory speed,
-# cheaper than unpacking every tile again inside the GEMM (measured on the gpt-oss-120b block:
-# 3.5 ms against 7.6 ms at 2048 rows, 5.1 ms at 8192 rows). Below the streaming kernel's range
-# nothing is left for the GEMM with unpack warps, so the default sends everything else here.
+# Above, packed 4-bit experts are expanded to bf16 once and run through the dense grouped GEMM: the
+# expansion is one pass over the layer's experts at memory speed, cheaper than unpacking every tile again
+# inside the GEMM (measured on the gpt-oss-120b block: 3.5 ms against 7.6 ms at 2048 rows, 5.1 ms at 8192
+# rows). Nothing is left for the GEMM with unpack warps, so the default sends everything else here.
+# gate/up and down of that block (us, streaming kernel / expansion and GEMM) at 16 rows an expert 768 and 418 /
+# 2246 and 1111, at 32 1230 and 677 / 2183 and 1128, at 64 2187 and 1193 / 2194 and 1153: the two meet at 64,
+# the limit of 16 was set when the streaming kernel took twice as long.
 _DEQUANT_MIN_ROWS = int(os.environ.get("MLXCEL_B200_MOE_DEQUANT_MIN_ROWS", "1"))
 
 

@@ -393,8 +393,9 @@ def qglu_linear(x: torch.Tensor, qt: QuantizedTensor, inter: int, act: str, bias
 
 
 def qlinear(x: torch.Tensor, qt: QuantizedTensor, bias=None, residual=None, out=None) -> torch.Tensor:
-    """``x @ dequant(w)^T (+ bias) (+ residual)``. M <= 8 rows stream the packed weights once
-    through the GEMV kernel; up to 256 rows go to the tcgen05 GEMM whose transform warps dequantise
+    """``x @ dequant(w)^T (+ bias) (+ residual)``. One row (up to ``MLXCEL_B200_QMV_MAX_M``; up to 8
+    of formats the fused GEMM does not take) streams the packed weights once through the GEMV
+    kernels; up to 256 rows go to the tcgen05 GEMM whose transform warps dequantise
     the packed tiles in shared memory (weights are read once, at 4 or 8 bits); larger M dequantizes
     into a reused bf16 buffer and runs the dense GEMM (prefill is compute bound, so the extra pass
     is small there)."""
